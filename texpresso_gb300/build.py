@@ -44,8 +44,10 @@ def _deps():
     return headers
 
 
-# Device code of the single-texture kernels (k_cluster, k_range, k_alpha).
-KERNEL_SOURCES = ("tx_alpha.cu", "tx_alpha.cuh", "tx_colour.cu", "tx_colour.cuh", "tx_device.cuh")
+# Device code of the single-texture kernels (k_cluster, k_cluster_lanes, k_range,
+# k_alpha).
+KERNEL_SOURCES = ("tx_alpha.cu", "tx_alpha.cuh", "tx_cluster_lanes.cu", "tx_cluster_lanes.cuh", "tx_colour.cu",
+                  "tx_colour.cuh", "tx_device.cuh")
 
 
 def source_digest():

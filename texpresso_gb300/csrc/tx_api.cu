@@ -120,6 +120,7 @@ int ensure_ready(DeviceState **out) {
     build_single_table(6, 4, lut[3]);
     cudaError_t e = tx::upload_colour_tables(lut);
     if (e != cudaSuccess) return fail(e);
+    if ((e = tx::upload_cluster_lane_tables(lut)) != cudaSuccess) return fail(e);
     if ((e = tx::upload_batch_tables(lut)) != cudaSuccess) return fail(e);
     for (int s = 0; s < kStreams; ++s) {
         if ((e = cudaStreamCreateWithFlags(&d.streams[s], cudaStreamNonBlocking)) != cudaSuccess) return fail(e);

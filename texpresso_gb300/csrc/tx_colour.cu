@@ -88,6 +88,18 @@ size_t cluster_smem_bytes(int team, int threads) {
 
 cudaError_t upload_colour_tables(const uint32_t lut[4][256][2]) { return upload_tables_this_tu(lut); }
 
+// SMs of the current device (0 if it cannot be asked), looked up once.
+static int device_sms() {
+    static int sm_count[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (sm_count[dev] == 0) {
+        int sms = 0;
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0) sm_count[dev] = sms;
+    }
+    return sm_count[dev];
+}
+
 template <int FMT>
 static cudaError_t launch_range_t(const SrcDesc &src, const DevParams &prm, uint8_t *out, size_t nblocks,
                                   cudaStream_t st, const LaunchCfg &cfg) {
@@ -109,18 +121,8 @@ static cudaError_t launch_cluster_t(const SrcDesc &src, const DevParams &prm, ui
     // its slot without waiting for CTA partners; the slowest SM sets the
     // launch's time.  (256x256 BC1: 25.9 us in one-warp CTAs, 26.5 us in
     // 2-team and 26.9 us in 4-team CTAs.)
-    static int sm_count[64] = {};
-    int dev0 = 0;
-    cudaGetDevice(&dev0);
-    if (dev0 < 64 && sm_count[dev0] == 0) {
-        int sms = 0;
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev0) == cudaSuccess && sms > 0)
-            sm_count[dev0] = sms;
-    }
     int threads = cfg.cluster_threads;
-    if (NITER == 1 && threads == 256 && dev0 < 64 && sm_count[dev0] > 0 &&
-        nblocks < (size_t)sm_count[dev0] * 4 * (256 / TEAM))
-        threads = 32;
+    if (NITER == 1 && threads == 256 && nblocks < (size_t)device_sms() * 4 * (256 / TEAM)) threads = 32;
     const size_t smem = cluster_smem_bytes(TEAM, threads);
     static bool attr_set[64] = {};
     int dev = 0;
@@ -188,6 +190,9 @@ cudaError_t launch_colour(int fmt, int algorithm, const SrcDesc &src, const DevP
         }
     }
     const bool iter = algorithm == ITERATIVE_CLUSTER_FIT;
+    if (!iter && !cluster_team_override() && cfg.cluster_team == 32 && cfg.max_ctas == LaunchCfg().max_ctas &&
+        cluster_lanes_take(fmt, prm, nblocks, device_sms()))
+        return launch_cluster_lanes(fmt, src, prm, out, nblocks, st);
     switch (fmt) {
     case BC1: return iter ? launch_cluster_team<BC1, 8>(src, prm, out, nblocks, st, cfg)
                           : launch_cluster_team<BC1, 1>(src, prm, out, nblocks, st, cfg);

@@ -2,7 +2,8 @@
 // the BC2/BC3 alpha halves, shared by the single-texture kernels (tx_colour.cu)
 // and the persistent batch kernel (tx_batch.cu).
 //
-// Two execution shapes:
+// Two execution shapes (and a third, for large ClusterFit launches of BC2 and BC3,
+// in tx_cluster_lanes.cuh):
 //   thread-per-block  ColourSet, SingleColourFit and RangeFit are short and
 //                     branch-light; a thread owns a block and 32 neighbouring
 //                     blocks load as four coalesced 512-byte rows.
@@ -203,15 +204,22 @@ __device__ __forceinline__ uint32_t dd_dup(const uint32_t (&res)[4], int i) {
     return (res[i >> 2] >> (8 * (i & 3) + 4)) & 0xFu;
 }
 
+// One thread's colour set (colourset.rs:35-141), pixel-indexed: a "point" is
+// the first pixel of its colour, and pixel order is point order.
+struct ColourSet {
+    uint32_t valid;    // pixels taking part
+    uint32_t newbits;  // pixels that are points
+    uint32_t dd[4];    // byte p: pixel p's point | (its colour's pixel count - 1) << 4
+    int count;         // points
+    bool transparent;
+};
+
 // px is overwritten with the colour-set keys (the RGB bytes of every valid
-// pixel are kept; alpha is not needed after the packed copy below), so the
-// pixels and the keys never occupy registers at the same time.
+// pixel are kept; alpha is not needed after the packed copy a4), so the pixels
+// and the keys never occupy registers at the same time.
 template <int FMT>
-__device__ __forceinline__ uint2 colour_range_thread(uint32_t (&px)[16], uint32_t inb,
-                                                     const DevParams &prm, const float *s_unorm,
-                                                     const float *s_sqrt, const PointCol &pt) {
-    // ColourSet (colourset.rs:35-112), pixel-indexed: a "point" is the first
-    // pixel of its colour, and pixel order is point order.
+__device__ __forceinline__ void colour_set_thread(uint32_t (&px)[16], uint32_t inb, bool alpha_weighted,
+                                                  uint32_t (&a4)[4], ColourSet &cs) {
     uint32_t tbits = 0;
     if (FMT == BC1) {
 #pragma unroll
@@ -219,44 +227,49 @@ __device__ __forceinline__ uint2 colour_range_thread(uint32_t (&px)[16], uint32_
         tbits &= inb;
     }
     const uint32_t valid = inb & ~tbits;
-    const bool transparent = tbits != 0;
-    uint32_t a4[4];  // alpha of pixel 4r + c at byte c of a4[r] (alpha weighting only)
-    if (prm.alpha_weighted) channel_words(px, 3, a4);
+    cs.valid = valid;
+    cs.transparent = tbits != 0;
+    if (alpha_weighted) channel_words(px, 3, a4);
 #pragma unroll
     for (int i = 0; i < 16; ++i) px[i] = ((valid >> i) & 1u) ? (px[i] & 0xFFFFFFu) : (0x01000000u | (uint32_t)i);
-    uint32_t dd[4];  // byte p: pixel p's point index | (its colour's pixel count - 1) << 4
-    colour_dedup(px, dd);
+    colour_dedup(px, cs.dd);
     // a valid pixel that is its own point starts a new point (excluded pixels
     // match nothing, so they are their own "point" too and are masked out)
     uint32_t newbits = 0;
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-        const uint32_t eq = bytes_eq(dd[w] & 0x0F0F0F0Fu, 0x03020100u + 0x04040404u * (uint32_t)w);
+        const uint32_t eq = bytes_eq(cs.dd[w] & 0x0F0F0F0Fu, 0x03020100u + 0x04040404u * (uint32_t)w);
         newbits |= (((eq & 0x08040201u) * 0x01010101u) >> 24) << (4 * w);
     }
-    newbits &= valid;
-    const int count = __popc(newbits);
+    cs.newbits = newbits & valid;
+    cs.count = __popc(cs.newbits);
+}
 
-    if (count == 1) {
-        uint32_t rgb = 0;
+// The block of a one-colour set (px as colour_set_thread leaves it).
+template <int FMT>
+__device__ __forceinline__ uint2 single_thread(const uint32_t (&px)[16], const ColourSet &cs, const float *s_unorm) {
+    uint32_t rgb = 0;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) rgb |= ((valid >> i) & 1u) ? px[i] : 0u;
-        int col[3];
+    for (int i = 0; i < 16; ++i) rgb |= ((cs.valid >> i) & 1u) ? px[i] : 0u;
+    int col[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) col[c] = f32_to_i32_clamped(s_unorm[u8_of(rgb, c)] * 255.0f, 255);
-        return single_fit<FMT>(col, valid, transparent);
-    }
+    for (int c = 0; c < 3; ++c) col[c] = f32_to_i32_clamped(s_unorm[u8_of(rgb, c)] * 255.0f, 255);
+    return single_fit<FMT>(col, cs.valid, cs.transparent);
+}
 
-    // Points and weights.  Pixels that are not points get weight exactly 0,
-    // which makes their terms +-0 in every ordered sum below.  Those sums start
-    // at +0 and add non-negative values (total, centroid) or can only reach
-    // zero as +0 (round-to-nearest x + (-x) = +0), so they are never -0 and
-    // adding +-0 leaves them unchanged: the sums equal the reference's sums
-    // over points.
-    if (!prm.alpha_weighted) {
+// Points and weights.  Pixels that are not points get weight exactly 0,
+// which makes their terms +-0 in every ordered sum below.  Those sums start
+// at +0 and add non-negative values (total, centroid) or can only reach
+// zero as +0 (round-to-nearest x + (-x) = +0), so they are never -0 and
+// adding +-0 leaves them unchanged: the sums equal the reference's sums
+// over points.
+__device__ __forceinline__ void colour_points_thread(const uint32_t (&px)[16], const uint32_t (&a4)[4],
+                                                     const ColourSet &cs, bool alpha_weighted, const float *s_unorm,
+                                                     const float *s_sqrt, const PointCol &pt) {
+    if (!alpha_weighted) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            const float w = ((newbits >> i) & 1u) ? s_sqrt[1 + (int)dd_dup(dd, i)] : 0.0f;
+            const float w = ((cs.newbits >> i) & 1u) ? s_sqrt[1 + (int)dd_dup(cs.dd, i)] : 0.0f;
             pt[i] = make_float4(s_unorm[u8_of(px[i], 0)], s_unorm[u8_of(px[i], 1)], s_unorm[u8_of(px[i], 2)], w);
         }
     } else {
@@ -269,18 +282,20 @@ __device__ __forceinline__ uint2 colour_range_thread(uint32_t (&px)[16], uint32_
             pt[j] = make_float4(s_unorm[u8_of(px[j], 0)], s_unorm[u8_of(px[j], 1)], s_unorm[u8_of(px[j], 2)], 0.0f);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            const float wa = ((valid >> i) & 1u)
+            const float wa = ((cs.valid >> i) & 1u)
                                  ? (float)(((a4[i >> 2] >> (8 * (i & 3))) & 0xFFu) + 1u) * (1.0f / 256.0f)
                                  : 0.0f;
-            float &w = pt[(int)dd_rep(dd, i)].w;
+            float &w = pt[(int)dd_rep(cs.dd, i)].w;
             w = w + wa;
         }
 #pragma unroll
         for (int j = 0; j < 16; ++j)
-            if ((newbits >> j) & 1u) pt[j].w = sqrt_rn(pt[j].w);
+            if ((cs.newbits >> j) & 1u) pt[j].w = sqrt_rn(pt[j].w);
     }
+}
 
-    // Sym3x3::weighted_covariance (math.rs:44-73)
+// Sym3x3::weighted_covariance (math.rs:44-73) of a thread's points.
+__device__ __forceinline__ void covariance_thread(const PointCol &pt, float (&m)[6]) {
     float total = 0.0f, cx = 0.0f, cy = 0.0f, cz = 0.0f;
 #pragma unroll 4
     for (int i = 0; i < 16; ++i) {
@@ -289,7 +304,8 @@ __device__ __forceinline__ uint2 colour_range_thread(uint32_t (&px)[16], uint32_
         cx = cx + q.x * q.w; cy = cy + q.y * q.w; cz = cz + q.z * q.w;
     }
     if (total > FLT_EPSILON) { cx = div_rn(cx, total); cy = div_rn(cy, total); cz = div_rn(cz, total); }
-    float m[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int c = 0; c < 6; ++c) m[c] = 0.0f;
 #pragma unroll 4
     for (int i = 0; i < 16; ++i) {
         const float4 q = pt[i];
@@ -298,6 +314,37 @@ __device__ __forceinline__ uint2 colour_range_thread(uint32_t (&px)[16], uint32_
         m[0] += ax * bx; m[1] += ax * by; m[2] += ax * bz;
         m[3] += ay * by; m[4] += ay * bz; m[5] += az * bz;
     }
+}
+
+// remap_indices (colourset.rs:130-141): 2-bit code of every point's pixel ->
+// code of every pixel, 3 for the excluded ones.  With 16 distinct valid
+// pixels every pixel is its own point and the map is the identity.
+__device__ __forceinline__ uint32_t remap_thread(const ColourSet &cs, uint32_t closest) {
+    if (cs.newbits == 0xFFFFu) return closest;
+    uint32_t out = 0;
+#pragma unroll
+    for (int p = 0; p < 16; ++p) {
+        const uint32_t r = dd_rep(cs.dd, p);
+        const uint32_t v = ((cs.valid >> p) & 1u) ? ((closest >> (2 * r)) & 3u) : 3u;
+        out |= v << (2 * p);
+    }
+    return out;
+}
+
+template <int FMT>
+__device__ __forceinline__ uint2 colour_range_thread(uint32_t (&px)[16], uint32_t inb,
+                                                     const DevParams &prm, const float *s_unorm,
+                                                     const float *s_sqrt, const PointCol &pt) {
+    uint32_t a4[4];  // alpha of pixel 4r + c at byte c of a4[r] (alpha weighting only)
+    ColourSet cs;
+    colour_set_thread<FMT>(px, inb, prm.alpha_weighted, a4, cs);
+    const uint32_t newbits = cs.newbits;
+    const int count = cs.count;
+    const bool transparent = cs.transparent;
+    if (count == 1) return single_thread<FMT>(px, cs, s_unorm);
+    colour_points_thread(px, a4, cs, prm.alpha_weighted, s_unorm, s_sqrt, pt);
+    float m[6];
+    covariance_thread(pt, m);
     float axis[3];
     principle_component(m, axis);
 
@@ -375,18 +422,7 @@ __device__ __forceinline__ uint2 colour_range_thread(uint32_t (&px)[16], uint32_
             err = err + (((newbits >> i) & 1u) ? dist : 0.0f);
         }
         if (err < best_err) {
-            // remap_indices (colourset.rs:130-141); with 16 distinct valid
-            // pixels every pixel is its own point and the map is the identity
-            uint32_t out = closest;
-            if (newbits != 0xFFFFu) {
-                out = 0;
-#pragma unroll
-                for (int p = 0; p < 16; ++p) {
-                    const uint32_t r = dd_rep(dd, p);
-                    const uint32_t v = ((valid >> p) & 1u) ? ((closest >> (2 * r)) & 3u) : 3u;
-                    out |= v << (2 * p);
-                }
-            }
+            const uint32_t out = remap_thread(cs, closest);
             indices = out;
             best_err = err;
             return true;

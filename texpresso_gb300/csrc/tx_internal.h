@@ -27,6 +27,12 @@ cudaError_t launch_colour(int fmt, int algorithm, const SrcDesc &src, const DevP
                           size_t nblocks, cudaStream_t st, const LaunchCfg &cfg);
 size_t cluster_smem_bytes(int team, int threads);
 
+// tx_cluster_lanes.cu: ClusterFit of BC2 and BC3 with one block per thread
+cudaError_t upload_cluster_lane_tables(const uint32_t lut[4][256][2]);
+bool cluster_lanes_take(int fmt, const DevParams &prm, size_t nblocks, int sm_count);  // whether it is to encode them
+cudaError_t launch_cluster_lanes(int fmt, const SrcDesc &src, const DevParams &prm, uint8_t *out, size_t nblocks,
+                                 cudaStream_t st);
+
 // tx_batch.cu
 cudaError_t upload_batch_tables(const uint32_t lut[4][256][2]);
 
