@@ -1,6 +1,14 @@
 // tx_api.cu -- the C ABI (include/texpresso_gb300.h): argument checks that
-// mirror the reference's panics, per-device state, and the host-buffer path
-// that streams an image through the GPU in bands of block rows so that the
+// mirror the reference's panics, per-device state, and the host-buffer calls.
+//
+// Host buffers.  On a Grace host the GPU reads and writes pageable memory
+// through the host's own page tables at the speed of the link, so the kernels
+// work on the caller's buffers (DeviceState::host_access): one launch, no copies.
+// A pageable copy makes the host wait for everything before it, so the bands
+// below ran one after another (1024x1024 from pageable memory: BC1 RangeFit 347
+// -> 46 us, BC1 ClusterFit of a smooth field 968 -> 584; BC3 ClusterFit 2048x2048
+// 1,228 -> 396 us, from pinned memory 767 -> 392; a 64x64 BC1 RangeFit 33 -> 25).
+// Elsewhere an image streams through the GPU in bands of block rows so that the
 // host->device copy of one band overlaps the kernel of the previous one.
 #include "texpresso_gb300.h"
 #include "tx_device.cuh"
@@ -36,6 +44,7 @@ struct DeviceState {
     uint8_t *d_out = nullptr;
     size_t out_cap = 0;
     int sm_count = 0;
+    bool host_access = false;           // kernels may use pageable host memory (host page tables)
 };
 
 DeviceState g_dev[kMaxDevices];
@@ -127,6 +136,10 @@ int ensure_ready(DeviceState **out) {
         if ((e = cudaEventCreateWithFlags(&d.joined[s], cudaEventDisableTiming)) != cudaSuccess) return fail(e);
     }
     if ((e = cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return fail(e);
+    int tables = 0;
+    if ((e = cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev)) != cudaSuccess)
+        return fail(e);
+    d.host_access = tables != 0;
     d.ready.store(1, std::memory_order_release);
     return TX_OK;
 }
@@ -170,6 +183,19 @@ cudaError_t launch_any(int format, int algorithm, const tx::SrcDesc &src, const 
     return tx::launch_colour(format, algorithm, src, dp, out, nblocks, st, cfg);
 }
 
+bool overlap(const uint8_t *a, size_t an, const uint8_t *b, size_t bn) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y ? an > y - x : bn > x - y;
+}
+
+// End of a host-buffer call: whatever failed, nothing may still run that uses
+// the caller's buffers when the call returns.
+int finish(cudaError_t e, cudaStream_t st) {
+    const cudaError_t done = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = done;
+    return e == cudaSuccess ? TX_OK : fail(e);
+}
+
 // Shared validation of Format::compress arguments (lib/src/lib.rs:287-303).
 int check_compress(int format, size_t width, size_t height, size_t output_len, size_t *nblocks) {
     if (!valid_format(format)) return TX_ERR_INVALID_FORMAT;
@@ -188,6 +214,11 @@ int check_compress(int format, size_t width, size_t height, size_t output_len, s
 int tx_internal_ensure_device() {
     DeviceState *d = nullptr;
     return ensure_ready(&d);
+}
+
+bool tx_internal_host_access() {
+    DeviceState *d = nullptr;
+    return ensure_ready(&d) == TX_OK && d->host_access;
 }
 
 void tx_internal_set_last_cuda_error(int err) { t_last_cuda = err; }
@@ -257,12 +288,34 @@ int tx_compress(int format, const uint8_t *rgba, size_t rgba_len, size_t width, 
         ~Range() { nvtxRangePop(); }
     } range;
     cudaError_t e;
-    if ((e = grow(&d->d_in, &d->in_cap, in_bytes ? in_bytes : 16)) != cudaSuccess) return fail(e);
-    if ((e = grow(&d->d_out, &d->out_cap, output_len)) != cudaSuccess) return fail(e);
-
     const size_t bs = tx_block_size(format), bw = tx_num_blocks(width);
     const size_t rows = (nblocks + bw - 1) / bw;  // output block rows (may exceed the image)
     const size_t pitch = 4 * width;
+    if (d->host_access) {
+        // Blocks are stored whole, so the output must be aligned to a block; and
+        // it must not share bytes with the image, which other warps still read.
+        // Otherwise one copy from device memory follows the kernel.
+        const bool direct = reinterpret_cast<uintptr_t>(output) % bs == 0 && !overlap(output, output_len, rgba, in_bytes);
+        if (!direct && (e = grow(&d->d_out, &d->out_cap, output_len)) != cudaSuccess) return fail(e);
+        uint8_t *out = direct ? output : d->d_out;
+        cudaStream_t st = d->streams[0];
+        tx::SrcDesc src;
+        src.base = rgba;
+        src.masks = nullptr;
+        src.pitch = pitch;
+        src.width = (uint32_t)width;
+        src.height = (uint32_t)height;
+        tx::set_blocks_wide(src, (uint32_t)bw);
+        src.channels = 4;
+        src.vec16 = (reinterpret_cast<uintptr_t>(rgba) % 16 == 0 && pitch % 16 == 0) ? 1 : 0;
+        src.mode = 0;
+        e = launch_any(format, algorithm, src, dp, out, nblocks, st);
+        if (e == cudaSuccess && !direct) e = cudaMemcpyAsync(output, out, output_len, cudaMemcpyDeviceToHost, st);
+        return finish(e, st);
+    }
+    if ((e = grow(&d->d_in, &d->in_cap, in_bytes ? in_bytes : 16)) != cudaSuccess) return fail(e);
+    if ((e = grow(&d->d_out, &d->out_cap, output_len)) != cudaSuccess) return fail(e);
+
     // Bands of block rows, each copied in, compressed and copied out on one of
     // the streams, so the copies of one band overlap the kernels of others.
     // Large images taper the bands (weights 1 4 8 8 8 8 8 4 1 of 50): the
@@ -332,23 +385,31 @@ int tx_compress_block_masked(int format, const uint8_t *rgba, uint32_t mask, con
     if ((rc = ensure_ready(&d)) != TX_OK) return rc;
     std::lock_guard<std::mutex> lk(d->mu);
     cudaError_t e;
-    if ((e = grow(&d->d_in, &d->in_cap, 128)) != cudaSuccess) return fail(e);
-    if ((e = grow(&d->d_out, &d->out_cap, 16)) != cudaSuccess) return fail(e);
-    uint8_t staging[68];
+    alignas(16) uint8_t staging[96];  // block, mask, encoded block
     std::memcpy(staging, rgba, 64);
     std::memcpy(staging + 64, &mask, 4);
     cudaStream_t st = d->streams[0];
-    if ((e = cudaMemcpyAsync(d->d_in, staging, 68, cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e);
+    const uint8_t *in = staging;
+    uint8_t *out = staging + 80;
+    if (!d->host_access) {
+        if ((e = grow(&d->d_in, &d->in_cap, 128)) != cudaSuccess) return fail(e);
+        if ((e = grow(&d->d_out, &d->out_cap, 16)) != cudaSuccess) return fail(e);
+        in = d->d_in;
+        out = d->d_out;
+        if ((e = cudaMemcpyAsync(d->d_in, staging, 68, cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e);
+    }
     tx::SrcDesc src;
     std::memset(&src, 0, sizeof(src));
-    src.base = d->d_in;
-    src.masks = reinterpret_cast<const uint32_t *>(d->d_in + 64);
+    src.base = in;
+    src.masks = reinterpret_cast<const uint32_t *>(in + 64);
     src.channels = 4;
     src.mode = 1;
-    if ((e = launch_any(format, algorithm, src, dp, d->d_out, 1, st)) != cudaSuccess) return fail(e);
-    if ((e = cudaMemcpyAsync(output, d->d_out, bs, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return fail(e);
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail(e);
-    return TX_OK;
+    e = launch_any(format, algorithm, src, dp, out, 1, st);
+    if (e == cudaSuccess && !d->host_access)
+        e = cudaMemcpyAsync(staging + 80, out, bs, cudaMemcpyDeviceToHost, st);
+    const int rc_done = finish(e, st);
+    if (rc_done == TX_OK) std::memcpy(output, staging + 80, bs);
+    return rc_done;
 }
 
 int tx_compress_device(int format, const void *src_ptr, size_t src_pitch, int channels, size_t width, size_t height,
@@ -429,20 +490,23 @@ int tx_decompress(int format, const uint8_t *data, size_t data_len, size_t width
     if (rc != TX_OK) return rc;
     std::lock_guard<std::mutex> lk(d->mu);
     cudaError_t e;
+    // blocks are read as 8-byte words; the output must not share bytes with them
     const size_t in_bytes = rows * bw * bs;
-    if ((e = grow(&d->d_in, &d->in_cap, in_bytes)) != cudaSuccess) return fail(e);
-    if ((e = grow(&d->d_out, &d->out_cap, output_len)) != cudaSuccess) return fail(e);
+    const bool read_host = d->host_access && reinterpret_cast<uintptr_t>(data) % 8 == 0;
+    const bool write_host = d->host_access && !(read_host && overlap(output, output_len, data, in_bytes));
     cudaStream_t st = d->streams[0];
-    if ((e = cudaMemcpyAsync(d->d_in, data, in_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e);
-    if ((e = tx::launch_decode(format, d->d_in, bw, rows, width, height, d->d_out, width * 4, output_len, st)) !=
-        cudaSuccess)
-        return fail(e);
+    if (!read_host) {
+        if ((e = grow(&d->d_in, &d->in_cap, in_bytes)) != cudaSuccess) return fail(e);
+        if ((e = cudaMemcpyAsync(d->d_in, data, in_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e);
+    }
+    if (!write_host && (e = grow(&d->d_out, &d->out_cap, output_len)) != cudaSuccess) return fail(e);
+    e = tx::launch_decode(format, read_host ? data : d->d_in, bw, rows, width, height, write_host ? output : d->d_out,
+                          width * 4, output_len, st);
     // every pixel of the first img_rows rows is written; bytes past them stay untouched
     const size_t written = img_rows * width * 4;
-    if (written && (e = cudaMemcpyAsync(output, d->d_out, written, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-        return fail(e);
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail(e);
-    return TX_OK;
+    if (e == cudaSuccess && !write_host && written)
+        e = cudaMemcpyAsync(output, d->d_out, written, cudaMemcpyDeviceToHost, st);
+    return finish(e, st);
 }
 
 int tx_decompress_block(int format, const uint8_t *block, size_t block_len, uint8_t *rgba) {
@@ -455,14 +519,23 @@ int tx_decompress_block(int format, const uint8_t *block, size_t block_len, uint
     if (rc != TX_OK) return rc;
     std::lock_guard<std::mutex> lk(d->mu);
     cudaError_t e;
-    if ((e = grow(&d->d_in, &d->in_cap, 16)) != cudaSuccess) return fail(e);
-    if ((e = grow(&d->d_out, &d->out_cap, 64)) != cudaSuccess) return fail(e);
     cudaStream_t st = d->streams[0];
-    if ((e = cudaMemcpyAsync(d->d_in, block, bs, cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e);
-    if ((e = tx::launch_decode(format, d->d_in, 1, 1, 4, 4, d->d_out, 16, 64, st)) != cudaSuccess) return fail(e);
-    if ((e = cudaMemcpyAsync(rgba, d->d_out, 64, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return fail(e);
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail(e);
-    return TX_OK;
+    alignas(16) uint8_t staging[80];  // block, pixels
+    std::memcpy(staging, block, bs);
+    const uint8_t *in = staging;
+    uint8_t *out = staging + 16;
+    if (!d->host_access) {
+        if ((e = grow(&d->d_in, &d->in_cap, 16)) != cudaSuccess) return fail(e);
+        if ((e = grow(&d->d_out, &d->out_cap, 64)) != cudaSuccess) return fail(e);
+        in = d->d_in;
+        out = d->d_out;
+        if ((e = cudaMemcpyAsync(d->d_in, staging, bs, cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e);
+    }
+    e = tx::launch_decode(format, in, 1, 1, 4, 4, out, 16, 64, st);
+    if (e == cudaSuccess && !d->host_access) e = cudaMemcpyAsync(staging + 16, out, 64, cudaMemcpyDeviceToHost, st);
+    const int rc_done = finish(e, st);
+    if (rc_done == TX_OK) std::memcpy(rgba, staging + 16, 64);
+    return rc_done;
 }
 
 int tx_decompress_device(int format, const void *data, size_t data_len, size_t width, size_t height, void *output,
