@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_teams(BatchQueue q) {
     __shared__ float s_sqrt[17];
     init_unorm_tables(s_unorm, s_sqrt);
     TeamSmem *teams = reinterpret_cast<TeamSmem *>(smem_raw);
-    const TeamTables tt{g_cand, g_cand + kCand4 + 1, s_unorm, s_sqrt};
+    const TeamTables tt{g_cand, s_unorm, s_sqrt};
     const Team<TEAM> tm;
     TeamSmem &sm = teams[threadIdx.x / TEAM];
 

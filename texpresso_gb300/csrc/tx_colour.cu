@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(256, 4) k_cluster(SrcDesc src, DevParams prm, 
         init_unorm_tables(s_unorm, s_sqrt);  // ends with __syncthreads
     }
     TeamSmem *teams = reinterpret_cast<TeamSmem *>(smem_raw);
-    const TeamTables tt{g_cand, g_cand + kCand4 + 1, NITER > 1 ? s_unorm : g_unorm8, NITER > 1 ? s_sqrt : g_sqrt_count};
+    const TeamTables tt{g_cand, NITER > 1 ? s_unorm : g_unorm8, NITER > 1 ? s_sqrt : g_sqrt_count};
     const Team<TEAM> tm;
     TeamSmem &sm = teams[threadIdx.x / TEAM];
     if (NITER == 1) {

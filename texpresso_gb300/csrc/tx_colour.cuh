@@ -10,9 +10,9 @@
 //   team-per-block    ClusterFit: a team of TEAM lanes (16 or 32) owns a block.
 //                     Lane p owns pixel p for ColourSet; the candidates (967
 //                     least-squares fits at 16 colours) are spread over the
-//                     team: each gets a lower bound of its error, only those
+//                     team: each gets a bound of its error, only those
 //                     the bound cannot exclude get the reference's exact error
-//                     (see cand_bound), and the lexicographic minimum on (error,
+//                     (see sweep4 and, for compress3, cand_bound), and the lexicographic minimum on (error,
 //                     position in the reference's loop order) selects exactly
 //                     the candidate the sequential "first strictly smaller
 //                     error" loop selects.
@@ -28,31 +28,32 @@ namespace tx {
 // packed start | end << 8 | error << 16.  Tables: 0 = 5_3, 1 = 6_3, 2 = 5_4, 3 = 6_4.
 static __constant__ uint32_t c_lut[4][256][2];
 
-// ClusterFit candidate lists.  Entry bits: 0-3 i (offset of S(0,i)),
-// 4-11 offset of S(i,j), 12-19 offset of S(j,k) (compress4 only),
-// 20-29 rank of (i,j[,k]) in the reference's loop order at 16 colours, so
-// comparing entries compares loop positions.
+// compress3's candidate list.  Entry bits: 0-3 i (offset of S(0,i)),
+// 4-11 offset of S(i,j), 20-29 rank of (i,j) in the reference's loop order at
+// 16 colours, so comparing entries compares loop positions.
 // Entries are sorted so that the first N[n] are exactly the candidates of an
-// n-colour set (those with max(i+1, j, k) <= n).
+// n-colour set (those with max(i+1, j) <= n).
 constexpr int kCand4 = 967, kCand3 = 151;
-static __device__ uint32_t g_cand[kCand4 + 1 + kCand3 + 1];
-static __constant__ uint32_t c_ncand4[17];
+static __device__ uint32_t g_cand[kCand3 + 1];
 static __constant__ uint32_t c_ncand3[17];
-// Positions, in the list an n-colour set uses, of its candidates with every
-// point in one cluster: compress4 (0,0,n) and (0,n,n), compress3 (0,n).
-static __constant__ uint16_t c_one4[17][2];
+// Position, in the list an n-colour set uses, of its candidate with every
+// point in one cluster, (0,n).
 static __constant__ uint16_t c_one3[17];
-// The same candidates in the reference's loop order (i, j, k nested), used for
+// The same candidates in the reference's loop order (i, j nested), used for
 // 16-colour sets: a round of consecutive candidates then mostly shares S(0,i)
-// and S(i,j) and reads S(j,k) at consecutive addresses.
-static __device__ uint32_t g_cand16[kCand4 + 1 + kCand3 + 1];
+// and reads S(i,j) at consecutive addresses.
+static __device__ uint32_t g_cand16[kCand3 + 1];
 // Lower-bound terms (F1, r, C, S offsets) of the g_cand16 candidates of a
 // 16-colour set whose weights are all exactly 1 (the w lanes of the partial
-// sums are then the counts i, j-i, k-j), from the reference's f32 alpha2,
+// sums are then the counts i, j-i), from the reference's f32 alpha2,
 // beta2, alphabeta (see unit_terms and unit_bound).  The w lane holds the
-// bits i | S(i,j) << 8 | S(j,k) << 16 (table offsets, one byte each).
-static __device__ float4 g_ub4[kCand4 + 1];
+// bits i | S(i,j) << 8 (table offsets, one byte each).
 static __device__ float4 g_ub3[kCand3 + 1];
+// The pairs (j, k), 0 <= j <= k <= n, k > 0, of compress4's candidates (i, j, k)
+// of an n-colour set, j | k << 5, j ascending: neighbouring pairs then take the
+// same i (0 .. min(j, n - 1)).
+constexpr int kPairs = 152;
+static __device__ uint16_t g_pairs[17][kPairs];
 // unorm8(v) for every byte v and sqrt(n) for n <= 16 (filled by k_unorm_tables
 // with the same correctly rounded division and square root as the kernels).
 static __device__ float g_unorm8[256];
@@ -481,8 +482,14 @@ struct Team {
     }
     __device__ __forceinline__ bool all(bool p) const { return __all_sync(mask, p); }
     template <class T> __device__ __forceinline__ T shfl(T v, int src) const { return __shfl_sync(mask, v, src, TEAM); }
+    template <class T> __device__ __forceinline__ T shfl_up(T v, int d) const { return __shfl_up_sync(mask, v, d, TEAM); }
     template <class T> __device__ __forceinline__ T shfl_xor(T v, int m) const { return __shfl_xor_sync(mask, v, m, TEAM); }
     __device__ __forceinline__ void sync() const { __syncwarp(mask); }
+    __device__ __forceinline__ float least(float v) const {
+        float r;
+        asm volatile("redux.sync.min.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "r"(mask));
+        return r;
+    }
     __device__ __forceinline__ unsigned match(uint32_t key) const {
         const unsigned m = __match_any_sync(mask, key);
         return (TEAM == 32) ? m : ((m >> base) & 0xFFFFu);
@@ -491,8 +498,11 @@ struct Team {
 
 struct __align__(16) TeamSmem {
     float4 S[kTri + 3];     // S(a,b) running sums at tri_idx(a,b) (+pad)
+    float4 Q[17];           // compress4: centred prefix sums and prefix weights of the ordering
+    float G[17];            // compress4: the bound's terms of i
     union {                 // lifetimes do not overlap within an iteration:
-        float LB[kCand4 + 1];   // candidate lower bounds, then the survivor queue
+        float LB[kCand3 + 9];   // compress3: candidate lower bounds, then the survivor queue; scratch
+        uint16_t queue[kCand4 + 1];  // compress4: the candidates to evaluate, i << 10 | j << 5 | k
         struct {
             float4 PW[16];      // points_weights in the current ordering
             uint32_t D[16];     // sort keys of the dot products
@@ -620,15 +630,14 @@ __device__ __forceinline__ float eval3(const float4 p0, const float4 p1, const f
     return fit_error<WANT_AB>(ax, bx, wt, cw, ea, eb);
 }
 
-// Decode (i, j, k) from a candidate entry.
-__host__ __device__ __forceinline__ void decode_entry(uint32_t e, int &i, int &j, int &k) {
+// Decode (i, j) from a candidate entry of compress3.
+__host__ __device__ __forceinline__ void decode_entry(uint32_t e, int &i, int &j) {
     i = (int)(e & 0xFu);
     j = (int)((e >> 4) & 0xFFu) - tri_idx(i, 0);
-    k = (int)((e >> 12) & 0xFFu) - tri_idx(j, 0);
 }
 
 // ---------------------------------------------------------------------------
-// Candidate pruning.  For a candidate with weight-lane terms alpha, beta,
+// Candidate pruning of compress3.  For a candidate with weight-lane terms alpha, beta,
 // gamma (> 0 definite) and per-channel sums ax, bx, the reference's error at
 // any endpoints (a, b) is  sum_c w_c Q_c(a_c, b_c)  with
 //     Q(a, b) = alpha a^2 + beta b^2 + 2 gamma a b - 2 a ax - 2 b bx
@@ -657,20 +666,11 @@ __host__ __device__ __forceinline__ void decode_entry(uint32_t e, int &i, int &j
 
 // Bound terms (A, -2B, alpha, 1/det) from the w lanes of the partial sums, for
 // blocks whose weights are not all 1 (no table entry applies).
-template <int NC>
-__device__ __forceinline__ float4 lb_terms(float p0w, float p1w, float p2w, float xsw) {
-    float al, be, g2;
-    if (NC == 4) {
-        const float p3w = xsw - p0w - p1w - p2w;
-        al = __fmaf_rn(p2w, 1.0f / 9.0f, __fmaf_rn(p1w, 4.0f / 9.0f, p0w));
-        be = __fmaf_rn(p1w, 1.0f / 9.0f, __fmaf_rn(p2w, 4.0f / 9.0f, p3w));
-        g2 = (4.0f / 9.0f) * (p1w + p2w);
-    } else {
-        const float p2r = xsw - p0w - p1w;
-        al = __fmaf_rn(p1w, 0.25f, p0w);
-        be = __fmaf_rn(p1w, 0.25f, p2r);
-        g2 = 0.5f * p1w;
-    }
+__device__ __forceinline__ float4 lb_terms(float p0w, float p1w, float xsw) {
+    const float p2r = xsw - p0w - p1w;
+    const float al = __fmaf_rn(p1w, 0.25f, p0w);
+    const float be = __fmaf_rn(p1w, 0.25f, p2r);
+    const float g2 = 0.5f * p1w;
     // det = al*be - g*g with the product g*g split exactly (its rounding error
     // recovered by an FMA), so det carries only the final roundings
     const float g = 0.5f * g2;
@@ -704,15 +704,12 @@ __device__ __forceinline__ BoundBlock bound_block(const float4 xs, const float (
 
 // -f (A sum w ax^2 - 2B sum w X ax + alpha Z + Kb) - eps1 for one candidate;
 // lt = (A, -2B, alpha, f).
-template <int NC>
-__device__ __forceinline__ float cand_bound(const float4 p0, const float4 p1, const float4 p2, const float4 lt,
+__device__ __forceinline__ float cand_bound(const float4 p0, const float4 p1, const float4 lt,
                                             const float (&cw)[3], const BoundBlock &bb) {
-    const float pa[3] = {p0.x, p0.y, p0.z}, pb[3] = {p1.x, p1.y, p1.z}, pc[3] = {p2.x, p2.y, p2.z};
+    const float pa[3] = {p0.x, p0.y, p0.z}, pb[3] = {p1.x, p1.y, p1.z};
     float ax[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-        ax[c] = (NC == 4) ? __fmaf_rn(pc[c], 1.0f / 3.0f, __fmaf_rn(pb[c], 2.0f / 3.0f, pa[c]))
-                          : __fmaf_rn(pb[c], 0.5f, pa[c]);
+    for (int c = 0; c < 3; ++c) ax[c] = __fmaf_rn(pb[c], 0.5f, pa[c]);
     float s1 = (cw[0] * ax[0]) * ax[0];
     s1 = __fmaf_rn(cw[1] * ax[1], ax[1], s1);
     s1 = __fmaf_rn(cw[2] * ax[2], ax[2], s1);
@@ -733,16 +730,13 @@ __device__ __forceinline__ float cand_bound(const float4 p0, const float4 p1, co
 // most 2 w_c X_c^2 in size and the sum carries at most ~10 u Z; with the
 // rounding of F1, r, C and the two final FMAs that is <= ~17 u f W Z, inside
 // the 26 u f W Z budgeted for the general form above.
-template <int NC>
-__device__ __forceinline__ float unit_bound(const float4 p0, const float4 p1, const float4 p2, const float4 q,
-                                            const float4 xs, const float (&cw)[3], const BoundBlock &bb) {
-    const float pa[3] = {p0.x, p0.y, p0.z}, pb[3] = {p1.x, p1.y, p1.z}, pc[3] = {p2.x, p2.y, p2.z};
+__device__ __forceinline__ float unit_bound(const float4 p0, const float4 p1, const float4 q, const float4 xs, const float (&cw)[3], const BoundBlock &bb) {
+    const float pa[3] = {p0.x, p0.y, p0.z}, pb[3] = {p1.x, p1.y, p1.z};
     const float X[3] = {xs.x, xs.y, xs.z};
     float sum = 0.0f;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const float ax = (NC == 4) ? __fmaf_rn(pc[c], 1.0f / 3.0f, __fmaf_rn(pb[c], 2.0f / 3.0f, pa[c]))
-                                   : __fmaf_rn(pb[c], 0.5f, pa[c]);
+        const float ax = __fmaf_rn(pb[c], 0.5f, pa[c]);
         const float d = __fmaf_rn(-q.y, X[c], ax);
         sum = c == 0 ? (cw[0] * ax) * d : __fmaf_rn(cw[c] * ax, d, sum);
     }
@@ -757,26 +751,160 @@ struct LaneBest {
     float a[3], b[3];
 };
 
-// Exact error and endpoints of the candidate entry e (cluster.rs:189-220,
-// :320-353), folded into the lane's best.
-template <int NC>
+// Exact error and endpoints of the compress3 candidate entry e (cluster.rs:189-220),
+// folded into the lane's best.
 __device__ __forceinline__ void eval_candidate(const TeamSmem &sm, uint32_t e, const float4 xs, const float (&cw)[3],
                                                LaneBest &lb) {
-    float a[3], b[3], err;
+    float a[3], b[3];
     const float4 p0 = sm.S[e & 0xFu];
     const float4 p1 = sm.S[(e >> 4) & 0xFFu];
-    if (NC == 4) {
-        const float4 p2 = sm.S[(e >> 12) & 0xFFu];
-        err = eval4<true>(p0, p1, p2, xs, wterms4(p0.w, p1.w, p2.w, xs.w), cw, a, b);
-    } else {
-        err = eval3<true>(p0, p1, xs, wterms3(p0.w, p1.w, xs.w), cw, a, b);
-    }
+    const float err = eval3<true>(p0, p1, xs, wterms3(p0.w, p1.w, xs.w), cw, a, b);
     if (err < lb.err || (err == lb.err && e < lb.ent)) {
         lb.err = err;
         lb.ent = e;
 #pragma unroll
         for (int c = 0; c < 3; ++c) { lb.a[c] = a[c]; lb.b[c] = b[c]; }
     }
+}
+
+// The same for compress4 candidate i << 10 | j << 5 | k (cluster.rs:315-372).
+__device__ __forceinline__ void eval_key(const TeamSmem &sm, uint32_t e, const float4 xs, const float (&cw)[3],
+                                         LaneBest &lb) {
+    float a[3], b[3];
+    const int i = (int)(e >> 10), j = (int)((e >> 5) & 31u), k = (int)(e & 31u);
+    const float4 p0 = sm.S[i], p1 = sm.S[tri_idx(i, j)], p2 = sm.S[tri_idx(j, k)];
+    const float err = eval4<true>(p0, p1, p2, xs, wterms4(p0.w, p1.w, p2.w, xs.w), cw, a, b);
+    if (err < lb.err || (err == lb.err && e < lb.ent)) {
+        lb.err = err;
+        lb.ent = e;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) { lb.a[c] = a[c]; lb.b[c] = b[c]; }
+    }
+}
+
+// compress4's candidates of one ordering of n points (cluster.rs:315-372): folds
+// them into the team's bests ob.  part: those that the bound excludes may be left
+// out; var: weighted variances per channel; guess: i | j << 5 | k << 10.
+//
+// A lane takes a pair (j, k) and all its i.  With Q(t), w(t) the centred prefix
+// sums and the prefix weights of the ordering, candidate (i, j, k) can only reach
+// an error of thr if
+//     s = |Q(i) + V|^2 / 2 + tol - c den >= 0,   V = Q(j) + Q(k)
+// (bound, c, den and rounding terms: tx_cluster_lanes.cuh), which is one addition
+// and four fused multiply-adds per candidate:
+//     s = P + G(i) + V . Q(i) + 2 c a w(i),   a = w(j) + w(k),
+//     P = |V|^2 / 2 + c (a (a - W) - 2 W w(j)) + tol,
+//     G(i) = |Q(i)|^2 / 2 + c w(i) (w(i) - 5 W).
+// Q is scaled by the square roots of the channel weights.  tol = 512 W T R covers
+// the 75 for these sums, the 204 for the prefixes and 16 for the scaling; eps is
+// the one for |a|, |b| <= 1 (121 W sum w_c R; 128 is taken).  Channel weights
+// below 2^-60 count as zero in the bound: all of their error, at most 128 w_c, is
+// in eps.  thr is the least error of the candidates around a guess.
+//
+// Bound by instruction issue and fetch, like all of the team form.  The bounds of
+// a block take 350 warp instructions and their set-up 200, where bounds from the
+// table S, a candidate per lane, with a division unless a table held the terms
+// for weights of 1, took 1,020 (1,490).  BC1 256x256 28.6 -> 22.2 us, 2048x2048
+// 969 -> 829, iterative 1,535 -> 1,338; BC3 900x900 of noisy ramps 155 -> 128,
+// of smooth fields 362 -> 352 (there nearly all candidates have to be evaluated).
+// A grid filter for such blocks (as in tx_cluster_lanes.cuh) cost the noisy ramps
+// 15 % in place and 6 % as a function of its own, for 9 % on smooth fields.
+template <int TEAM>
+__device__ __forceinline__ void sweep4(const Team<TEAM> &tm, TeamSmem &sm, int n, const float4 xs, const float (&cw)[3],
+                                       const float (&var)[3], bool part, uint32_t guess, LaneBest &ob) {
+    const int lane = tm.lane;
+    float c = 0.f, tol = 0.f;
+    if (part) {
+        const int gi = (int)(guess & 31u), gj = (int)((guess >> 5) & 31u), gk = (int)(guess >> 10);
+#pragma unroll 1
+        for (int t = lane; t < 32; t += TEAM) {
+            const int t3 = t * 11 >> 5, t9 = t * 57 >> 9;  // t / 3, t / 9
+            const int i = min(max(gi + (t - 3 * t3) - 1, 0), n - 1);
+            const int j = min(max(gj + (t3 - 3 * t9) - 1, i), n);
+            const int k = min(max(gk + t9 - 1, max(j, 1)), n);
+            eval_key(sm, (uint32_t)(i << 10 | j << 5 | k), xs, cw, ob);
+        }
+        const float thr = tm.least(ob.err);
+        float T = 0.f, z = 0.f, sum = 0.f, tiny = 0.f, sq[3];
+        const float X[3] = {xs.x, xs.y, xs.z};
+#pragma unroll
+        for (int h = 0; h < 3; ++h) {
+            const float w = cw[h] < 0x1p-60f ? 0.0f : cw[h];
+            tiny += cw[h] - w;
+            sum += w;
+            z = __fmaf_rn(w * X[h], X[h], z);
+            T = __fmaf_rn(w, var[h], T);
+            asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(sq[h]) : "f"(w));
+        }
+        const float W = xs.w;
+        float rw;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rw) : "f"(W));
+        // the gain a candidate needs for thr, and c = gain / (2 W)
+        const float g = -__fmaf_rn(z, rw, thr) - __fmaf_rn(0x1p-17f * W, sum, 128.0f * tiny);
+        c = g > 0.0f ? g * (0.4999995f * rw) : 0.0f;
+        tol = __fmaf_rn(0x1.03p-15f * W, T, 1e-30f);  // 512 R W T
+        // centred weighted point of position `lane`, and the sums up to it
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (lane < n) q = sm.S[tri_idx(lane, 0) + lane + 1];
+        q.x = __fmaf_rn(-X[0] * rw, q.w, q.x) * sq[0];
+        q.y = __fmaf_rn(-X[1] * rw, q.w, q.y) * sq[1];
+        q.z = __fmaf_rn(-X[2] * rw, q.w, q.z) * sq[2];
+#pragma unroll
+        for (int off = 1; off < 16; off <<= 1) {
+            const float x = tm.shfl_up(q.x, off), y = tm.shfl_up(q.y, off), z1 = tm.shfl_up(q.z, off);
+            if (lane >= off) { q.x += x; q.y += y; q.z += z1; }
+        }
+        if (lane < n) {
+            q.w = sm.S[lane + 1].w;
+            sm.Q[lane + 1] = q;
+            const float h = __fmaf_rn(q.x, q.x, __fmaf_rn(q.y, q.y, q.z * q.z));
+            sm.G[lane + 1] = __fmaf_rn(c * q.w, __fmaf_rn(-5.0f, W, q.w), 0.5f * h);
+        }
+        if (lane == 0) {
+            sm.Q[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+            sm.G[0] = 0.0f;
+        }
+        tm.sync();
+    }
+    const int pairs = (n + 1) * (n + 2) / 2 - 1;
+    const unsigned below = (1u << lane) - 1u;
+    uint32_t nq = 0;
+#pragma unroll 1
+    for (int p0 = 0; p0 < pairs; p0 += TEAM) {
+        const int p = p0 + lane;
+        const uint32_t jk = __ldg(&g_pairs[n][min(p, pairs - 1)]);
+        const int j = (int)(jk & 31u), k = (int)(jk >> 5);
+        uint32_t keep = p < pairs ? (2u << min(j, n - 1)) - 1u : 0u;  // bit i: candidate (i, j, k)
+        if (part) {
+            const float4 qj = sm.Q[j], qk = sm.Q[k];
+            const float vx = qj.x + qk.x, vy = qj.y + qk.y, vz = qj.z + qk.z, a = qj.w + qk.w;
+            const float ca = c * a;
+            float P = __fmaf_rn(0.5f, __fmaf_rn(vx, vx, __fmaf_rn(vy, vy, vz * vz)), tol);
+            P = __fmaf_rn(ca, a - xs.w, P);
+            P = __fmaf_rn(-2.0f * c * xs.w, qj.w, P);
+            const float ca2 = 2.0f * ca;
+            uint32_t out = 0;  // signs of s, i descending
+#pragma unroll 1
+            for (int i = min(tm.shfl(j, TEAM - 1), n - 1) | 1; i > 0; i -= 2) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float4 q = sm.Q[i - h];
+                    const float s = __fmaf_rn(vx, q.x, __fmaf_rn(vy, q.y, __fmaf_rn(vz, q.z, __fmaf_rn(ca2, q.w, P + sm.G[i - h]))));
+                    out = __funnelshift_l(__float_as_uint(s), out, 1);
+                }
+            }
+            keep &= ~out;
+        }
+        // pack what is left, one i of every pair at a time
+        for (unsigned b = tm.ballot(keep != 0u); b != 0u; b = tm.ballot(keep != 0u)) {
+            if (keep) sm.queue[nq + __popc(b & below)] = (uint16_t)((__ffs(keep) - 1) << 10 | j << 5 | k);
+            keep &= keep - 1u;
+            nq += (uint32_t)__popc(b);
+        }
+    }
+    tm.sync();
+#pragma unroll 1
+    for (uint32_t t = (uint32_t)lane; t < nq; t += TEAM) eval_key(sm, sm.queue[t], xs, cw, ob);
 }
 
 // The ordering along the principal axis is the first ordering of both
@@ -787,19 +915,21 @@ struct SharedOrder {
     bool valid;  // S and hist[0] hold the principal-axis ordering
     int rank;    // this lane's point's position in it
     bool finite; // every dot product was finite
+    uint32_t guess;  // points before 1/6, 1/2 and 5/6 of the projections' range (sweep4)
 };
 
 // ClusterFit::compress3 / compress4 (cluster.rs:152-417) for one team.
 // best_err / best carry the ColourFit state across compress3 -> compress4.
 // LEAN (BC1 IterativeClusterFit, whose two passes make the largest kernel and
 // whose top stall is instruction fetch) trades unrolling for code size: the
-// rank and partial-sum loops are unrolled 4 times instead of 16, and short
-// lists go through the survivor sweep instead of a sweep of their own
-// (1,557 vs 1,604 us for 2048x2048; the other kernels measured faster
+// rank and partial-sum loops are unrolled 4 times instead of 16, and compress3's
+// short lists go through the survivor sweep instead of a sweep of their own
+// (1,557 vs 1,604 us for 2048x2048 when measured; the other kernels were faster
 // without these changes).
 template <int NC, int TEAM, int NITER, bool LEAN = false>
 __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm, const uint32_t *tbl, int count,
                                              const float (&principal)[3], const float (&cw)[3], bool prune,
+                                             const float (&var)[3],
                                              bool valid, int my_point, bool unit16, float &best_err, uint2 &best,
                                              SharedOrder &so) {
     const int lane = tm.lane;
@@ -809,7 +939,7 @@ __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm,
     int bit = 0, best_rank = 0;
     bool best_finite = false;
     float axis[3] = {principal[0], principal[1], principal[2]};
-    const uint32_t ncand = (NC == 4) ? c_ncand4[count] : c_ncand3[count];
+    const uint32_t ncand = (NC == 4) ? 0u : c_ncand3[count];
     float4 xs = make_float4(0.f, 0.f, 0.f, 0.f);
 
 #pragma unroll 1
@@ -817,13 +947,24 @@ __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm,
         // construct_ordering (cluster.rs:78-136)
         int my_rank = 0;
         bool finite;
+        uint32_t guess;
         if (NITER == 1 && so.valid) {  // (the iterative kernel measured faster rebuilding it)
             my_rank = so.rank;
             finite = so.finite;
+            guess = so.guess;
         } else {
             float de = FLT_MAX;
             if (lane < count) de = sm.P[0][lane] * axis[0] + sm.P[1][lane] * axis[1] + sm.P[2][lane] * axis[2];
             const uint32_t ke = dps_key(de);
+            {
+                const bool p = lane < count;
+                const uint32_t k0 = __reduce_min_sync(tm.mask, ke), k1 = __reduce_max_sync(tm.mask, p ? ke : 0u);
+                auto value = [](uint32_t k) { return __uint_as_float(k ^ (~(uint32_t)((int32_t)k >> 31) | 0x80000000u)); };
+                const float d0 = value(k0), r = value(k1) - d0;
+                guess = (uint32_t)__popc(tm.ballot(p && de < __fmaf_rn(r, 1.0f / 6.0f, d0))) |
+                        (uint32_t)__popc(tm.ballot(p && de < __fmaf_rn(r, 0.5f, d0))) << 5 |
+                        (uint32_t)__popc(tm.ballot(p && de < __fmaf_rn(r, 5.0f / 6.0f, d0))) << 10;
+            }
             if (lane < 16) sm.D[lane] = ke;
             tm.sync();
             if (lane < 16) {
@@ -891,6 +1032,7 @@ __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm,
             so.valid = it == 0;
             so.rank = my_rank;
             so.finite = finite;
+            so.guess = guess;
         }
         xs = sm.S[count];  // S(0, count) == xsum_wsum
 
@@ -903,7 +1045,10 @@ __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm,
 #pragma unroll
         for (int c = 0; c < 3; ++c) { ob.a[c] = 0.0f; ob.b[c] = 0.0f; }
         uint32_t lean_nq = 0;  // LEAN: candidates queued for the exact sweep below
-        if (ncand <= 2u * TEAM || !prune) {
+        if constexpr (NC == 4) {
+            // (up to 5 points have 54 candidates)
+            sweep4(tm, sm, count, xs, cw, var, prune && finite && count > 5, guess, ob);
+        } else if (ncand <= 2u * TEAM || !prune) {
             if (LEAN) {
                 uint32_t *queue = reinterpret_cast<uint32_t *>(sm.LB);
                 for (uint32_t t = (uint32_t)lane; t < ncand; t += TEAM) queue[t] = t;
@@ -911,7 +1056,7 @@ __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm,
                 tm.sync();
             } else {
                 // short lists: the plain sweep, lane-strided over the candidates
-                for (uint32_t t = (uint32_t)lane; t < ncand; t += TEAM) eval_candidate<NC>(sm, __ldg(tbl + t), xs, cw, ob);
+                for (uint32_t t = (uint32_t)lane; t < ncand; t += TEAM) eval_candidate(sm, __ldg(tbl + t), xs, cw, ob);
             }
         } else {
             // 1. a lower bound of every candidate's error (see cand_bound)
@@ -919,15 +1064,14 @@ __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm,
             float lmin = __int_as_float(0x7f800000);
             uint32_t tseed = 0xFFFFFFFFu;
             if (unit16) {
-                const float4 *ub = (NC == 4 ? g_ub4 : g_ub3) + lane;
+                const float4 *ub = g_ub3 + lane;
 #pragma unroll (NITER > 1 ? 1 : 2)
                 for (uint32_t t = (uint32_t)lane; t < ncand; t += TEAM, ub += TEAM) {
                     const float4 q = __ldg(ub);
                     const uint32_t o = __float_as_uint(q.w);
                     const float4 p0 = sm.S[o & 0xFFu];
                     const float4 p1 = sm.S[(o >> 8) & 0xFFu];
-                    const float4 p2 = (NC == 4) ? sm.S[o >> 16] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    const float bnd = unit_bound<NC>(p0, p1, p2, q, xs, cw, bb);
+                    const float bnd = unit_bound(p0, p1, q, xs, cw, bb);
                     sm.LB[t] = bnd;
                     if (bnd < lmin) { lmin = bnd; tseed = t; }
                 }
@@ -937,8 +1081,7 @@ __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm,
                     const uint32_t e = __ldg(tbl + t);
                     const float4 p0 = sm.S[e & 0xFu];
                     const float4 p1 = sm.S[(e >> 4) & 0xFFu];
-                    const float4 p2 = (NC == 4) ? sm.S[(e >> 12) & 0xFFu] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    const float bnd = cand_bound<NC>(p0, p1, p2, lb_terms<NC>(p0.w, p1.w, p2.w, xs.w), cw, bb);
+                    const float bnd = cand_bound(p0, p1, lb_terms(p0.w, p1.w, xs.w), cw, bb);
                     sm.LB[t] = bnd;
                     if (bnd < lmin) { lmin = bnd; tseed = t; }
                 }
@@ -946,7 +1089,7 @@ __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm,
             // 2. seeds: every lane's smallest bound, evaluated exactly; the
             // threshold is the smallest error reached (never above run)
             if (tseed != 0xFFFFFFFFu) {
-                eval_candidate<NC>(sm, __ldg(tbl + tseed), xs, cw, ob);
+                eval_candidate(sm, __ldg(tbl + tseed), xs, cw, ob);
                 sm.LB[tseed] = __int_as_float(0x7f800000);  // already evaluated
             }
             const uint32_t ngroups = (ncand + 3u) >> 2;
@@ -962,17 +1105,10 @@ __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm,
                     float rw;
                     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rw) : "f"(xs.w));
                     const float flat = __fmaf_rn(-(1.0f + 0x1p-10f) * bb.z, rw, -bb.eps1);
-                    if (NC == 4) {
-                        sm.LB[c_one4[count][0]] = flat;
-                        sm.LB[c_one4[count][1]] = flat;
-                    } else {
-                        sm.LB[c_one3[count]] = flat;
-                    }
+                    sm.LB[c_one3[count]] = flat;
                 }
             }
-            float thr = ob.err;
-#pragma unroll
-            for (int off = TEAM / 2; off > 0; off >>= 1) thr = fminf(thr, tm.shfl_xor(thr, off));
+            const float thr = tm.least(ob.err);
             tm.sync();
             // 3. survivors (bound not above thr; NaN = no bound) are packed in
             // place into the front of LB, four bounds per lane and round; a
@@ -1001,22 +1137,16 @@ __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm,
             if (LEAN)
                 lean_nq = nq;
             else
-                for (uint32_t s = (uint32_t)lane; s < nq; s += TEAM) eval_candidate<NC>(sm, __ldg(tbl + queue[s]), xs, cw, ob);
+                for (uint32_t s = (uint32_t)lane; s < nq; s += TEAM) eval_candidate(sm, __ldg(tbl + queue[s]), xs, cw, ob);
         }
-        if (LEAN) {
+        if (LEAN && NC == 3) {
             const uint32_t *queue = reinterpret_cast<const uint32_t *>(sm.LB);
-            for (uint32_t s = (uint32_t)lane; s < lean_nq; s += TEAM) eval_candidate<NC>(sm, __ldg(tbl + queue[s]), xs, cw, ob);
+            for (uint32_t s = (uint32_t)lane; s < lean_nq; s += TEAM) eval_candidate(sm, __ldg(tbl + queue[s]), xs, cw, ob);
         }
         // lexicographic reduction of the lanes' bests; the winning lane (the
         // one holding the winning entry) supplies the endpoints
-        float lbest = ob.err;
-        uint32_t lent = ob.ent;
-#pragma unroll
-        for (int off = TEAM / 2; off > 0; off >>= 1) {
-            const float oe = tm.shfl_xor(lbest, off);
-            const uint32_t on = tm.shfl_xor(lent, off);
-            if (oe < lbest || (oe == lbest && on < lent)) { lbest = oe; lent = on; }
-        }
+        const float lbest = tm.least(ob.err);
+        const uint32_t lent = __reduce_min_sync(tm.mask, ob.err == lbest ? ob.ent : 0xFFFFFFFFu);
         if (lent != 0u) {
             const int src = __ffs(tm.ballot(ob.ent == lent)) - 1;
 #pragma unroll
@@ -1034,7 +1164,14 @@ __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm,
 
     if (run < best_err) {
         int i, j, k;
-        decode_entry(bentry, i, j, k);
+        if (NC == 4) {
+            i = (int)(bentry >> 10);
+            j = (int)((bentry >> 5) & 31u);
+            k = (int)(bentry & 31u);
+        } else {
+            decode_entry(bentry, i, j);
+            k = 16;
+        }
         uint32_t ind = 3;
         // position of this pixel's point in the winning ordering: its rank, or
         // (with non-finite dot products) the last position < count holding it
@@ -1057,14 +1194,14 @@ __device__ __forceinline__ void cluster_pass(const Team<TEAM> &tm, TeamSmem &sm,
 // Per-CTA inputs of the team path: the candidate lists for sets of fewer than
 // 16 colours and the exact u8 -> [0,1] and sqrt(count) tables in shared memory.
 struct TeamTables {
-    const uint32_t *cand4, *cand3;
+    const uint32_t *cand3;
     const float *unorm, *sqrt;
 };
 
 template <int FMT, int TEAM, int NITER>
 __device__ __forceinline__ uint2 colour_cluster_team(const Team<TEAM> &tm, TeamSmem &sm, const TeamTables &tt,
                                                      uint32_t px, bool inb, const DevParams &prm) {
-    const uint32_t *tbl4 = tt.cand4, *tbl3 = tt.cand3;
+    const uint32_t *tbl3 = tt.cand3;
     const int lane = tm.lane;
     const uint32_t a = px >> 24;
     const bool tr = (FMT == BC1) && inb && a < 128u;
@@ -1163,19 +1300,22 @@ __device__ __forceinline__ uint2 colour_cluster_team(const Team<TEAM> &tm, TeamS
     uint2 best = make_uint2(0u, 0u);
     // 16 distinct colours without alpha weighting: every weight is sqrt(1) = 1
     const bool unit16 = count == 16 && !prm.alpha_weighted;
-    if (count == 16) { tbl4 = g_cand16; tbl3 = g_cand16 + kCand4 + 1; }
+    if (count == 16) tbl3 = g_cand16;
     // the error bound used for pruning holds for finite, non-negative weights
     const bool prune = cw[0] >= 0.0f && cw[1] >= 0.0f && cw[2] >= 0.0f && cw[0] <= FLT_MAX && cw[1] <= FLT_MAX &&
                        cw[2] <= FLT_MAX;
-    SharedOrder so{false, 0, false};
+    // compress4's bound: ordinary weights (products of larger ones leave the f32 range)
+    const bool part = prune && cw[0] <= 0x1p60f && cw[1] <= 0x1p60f && cw[2] <= 0x1p60f;
+    const float var[3] = {cov[0], cov[3], cov[5]};
+    SharedOrder so{false, 0, false, 0u};
     if (FMT == BC1) {
-        cluster_pass<3, TEAM, NITER, (NITER > 1)>(tm, sm, tbl3, count, principal, cw, prune, valid, my_point, unit16, best_err,
+        cluster_pass<3, TEAM, NITER, (NITER > 1)>(tm, sm, tbl3, count, principal, cw, prune, var, valid, my_point, unit16, best_err,
                                      best, so);
         if (!transparent)
-            cluster_pass<4, TEAM, NITER, (NITER > 1)>(tm, sm, tbl4, count, principal, cw, prune, valid, my_point, unit16, best_err,
+            cluster_pass<4, TEAM, NITER, (NITER > 1)>(tm, sm, nullptr, count, principal, cw, part, var, valid, my_point, unit16, best_err,
                                          best, so);
     } else {
-        cluster_pass<4, TEAM, NITER>(tm, sm, tbl4, count, principal, cw, prune, valid, my_point, unit16, best_err,
+        cluster_pass<4, TEAM, NITER>(tm, sm, nullptr, count, principal, cw, part, var, valid, my_point, unit16, best_err,
                                      best, so);
     }
     return best;
@@ -1356,21 +1496,14 @@ __device__ __forceinline__ float4 unit_terms(const float4 w, uint32_t offs, bool
                        __uint_as_float(offs));
 }
 
-// Fill the bound terms g_ub4 / g_ub3 from this TU's loop-order candidate
-// lists: the w-lane sums of a 16-point, weight-1 set are S(a,b).w = b - a
-// (exact small integers), and wterms4 / wterms3 are the reference's f32 code.
+// Fill the bound terms g_ub3 from this TU's loop-order candidate
+// list: the w-lane sums of a 16-point, weight-1 set are S(a,b).w = b - a
+// (exact small integers), and wterms3 is the reference's f32 code.
 static __global__ void k_unit_terms() {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < kCand4) {
-        int i, j, k;
-        decode_entry(g_cand16[t], i, j, k);
-        const uint32_t offs = (uint32_t)tri_idx(0, i) | (uint32_t)tri_idx(i, j) << 8 | (uint32_t)tri_idx(j, k) << 16;
-        const bool one = (i == 16) + (j - i == 16) + (k - j == 16) + (16 - k == 16) == 1;
-        g_ub4[t] = unit_terms(wterms4((float)i, (float)(j - i), (float)(k - j), 16.0f), offs, one);
-    }
     if (t < kCand3) {
-        int i, j, k;
-        decode_entry(g_cand16[kCand4 + 1 + t], i, j, k);
+        int i, j;
+        decode_entry(g_cand16[t], i, j);
         const uint32_t offs = (uint32_t)tri_idx(0, i) | (uint32_t)tri_idx(i, j) << 8;
         const bool one = (i == 16) + (j - i == 16) + (16 - j == 16) == 1;
         g_ub3[t] = unit_terms(wterms3((float)i, (float)(j - i), 16.0f), offs, one);
@@ -1383,20 +1516,10 @@ static __global__ void k_unit_terms() {
 // Build the candidate lists and single-colour tables and copy them to the
 // current device.
 static inline cudaError_t upload_tables_this_tu(const uint32_t lut[4][256][2]) {
-    // compress4: (i, j, k), 0 <= i < 16, i <= j <= 16, max(j,1) <= k <= 16
+    // compress3: (i, j), 0 <= i < 16, max(i,1) <= j <= 16
     struct C { int m, rank; uint32_t e; };
-    C c4[kCand4], c3[kCand3];
-    int n4 = 0, n3 = 0;
-    for (int i = 0; i < 16; ++i)
-        for (int j = i; j <= 16; ++j)
-            for (int k = (j == 0 ? 1 : j); k <= 16; ++k) {
-                const int m = (i + 1 > j ? i + 1 : j) > k ? (i + 1 > j ? i + 1 : j) : k;
-                c4[n4].m = m;
-                c4[n4].rank = n4;
-                c4[n4].e = (uint32_t)i | ((uint32_t)tri_idx(i, j) << 4) | ((uint32_t)tri_idx(j, k) << 12) |
-                           ((uint32_t)n4 << 20);
-                ++n4;
-            }
+    C c3[kCand3];
+    int n3 = 0;
     for (int i = 0; i < 16; ++i)
         for (int j = (i == 0 ? 1 : i); j <= 16; ++j) {
             const int m = i + 1 > j ? i + 1 : j;
@@ -1405,51 +1528,38 @@ static inline cudaError_t upload_tables_this_tu(const uint32_t lut[4][256][2]) {
             c3[n3].e = (uint32_t)i | ((uint32_t)tri_idx(i, j) << 4) | ((uint32_t)n3 << 20);
             ++n3;
         }
-    if (n4 != kCand4 || n3 != kCand3) return cudaErrorInvalidValue;
-    uint32_t loop_tbl[kCand4 + 1 + kCand3 + 1] = {};
-    for (int t = 0; t < kCand4; ++t) loop_tbl[t] = c4[t].e;
-    for (int t = 0; t < kCand3; ++t) loop_tbl[kCand4 + 1 + t] = c3[t].e;
-    auto sort_by_m = [](C *v, int n) {
-        for (int a = 1; a < n; ++a) {  // stable insertion sort on m
-            C t = v[a];
-            int b = a;
-            while (b > 0 && v[b - 1].m > t.m) { v[b] = v[b - 1]; --b; }
-            v[b] = t;
-        }
-    };
-    sort_by_m(c4, n4);
-    sort_by_m(c3, n3);
-    uint32_t tbl[kCand4 + 1 + kCand3 + 1] = {};
-    uint32_t nc4[17] = {}, nc3[17] = {};
-    for (int t = 0; t < kCand4; ++t) tbl[t] = c4[t].e;
-    for (int t = 0; t < kCand3; ++t) tbl[kCand4 + 1 + t] = c3[t].e;
-    for (int n = 0; n <= 16; ++n) {
-        for (int t = 0; t < kCand4; ++t) nc4[n] += c4[t].m <= n ? 1u : 0u;
+    if (n3 != kCand3) return cudaErrorInvalidValue;
+    uint32_t loop_tbl[kCand3 + 1] = {}, tbl[kCand3 + 1] = {}, nc3[17] = {};
+    for (int t = 0; t < kCand3; ++t) loop_tbl[t] = c3[t].e;
+    for (int a = 1; a < n3; ++a) {  // stable insertion sort on m
+        C t = c3[a];
+        int b = a;
+        while (b > 0 && c3[b - 1].m > t.m) { c3[b] = c3[b - 1]; --b; }
+        c3[b] = t;
+    }
+    for (int t = 0; t < kCand3; ++t) tbl[t] = c3[t].e;
+    for (int n = 0; n <= 16; ++n)
         for (int t = 0; t < kCand3; ++t) nc3[n] += c3[t].m <= n ? 1u : 0u;
+    // position of the one-cluster candidate in the list each count uses
+    uint16_t one3[17] = {};
+    for (int n = 1; n <= 16; ++n) {
+        const uint32_t *list = n == 16 ? loop_tbl : tbl;
+        for (int t = 0; t < kCand3; ++t)
+            if ((list[t] & 0xFFFu) == (uint32_t)tri_idx(0, n) << 4) one3[n] = (uint16_t)t;  // the i and S(i,j) fields
+    }
+    uint16_t pairs[17][kPairs] = {};
+    for (int n = 1; n <= 16; ++n) {
+        int t = 0;
+        for (int j = 0; j <= n; ++j)
+            for (int k = j == 0 ? 1 : j; k <= n; ++k) pairs[n][t++] = (uint16_t)(j | k << 5);
     }
     cudaError_t e;
     if ((e = cudaMemcpyToSymbol(g_cand, tbl, sizeof(tbl))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(g_cand16, loop_tbl, sizeof(loop_tbl))) != cudaSuccess) return e;
-    if ((e = cudaMemcpyToSymbol(c_ncand4, nc4, sizeof(nc4))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(c_ncand3, nc3, sizeof(nc3))) != cudaSuccess) return e;
-    // positions of the one-cluster candidates in the list each count uses
-    uint16_t one4[17][2] = {}, one3[17] = {};
-    auto find = [](const uint32_t *list, int n, uint32_t key, uint32_t mask) {
-        for (int t = 0; t < n; ++t)
-            if ((list[t] & mask) == key) return (uint16_t)t;
-        return (uint16_t)0;
-    };
-    for (int n = 1; n <= 16; ++n) {
-        const uint32_t *l4 = n == 16 ? loop_tbl : tbl;
-        const uint32_t *l3 = n == 16 ? loop_tbl + kCand4 + 1 : tbl + kCand4 + 1;
-        const uint32_t m4 = 0xFFFFFu, m3 = 0xFFFu;  // the i, S(i,j), S(j,k) fields
-        one4[n][0] = find(l4, kCand4, (uint32_t)tri_idx(0, 0) << 4 | (uint32_t)tri_idx(0, n) << 12, m4);
-        one4[n][1] = find(l4, kCand4, (uint32_t)tri_idx(0, n) << 4 | (uint32_t)tri_idx(n, n) << 12, m4);
-        one3[n] = find(l3, kCand3, (uint32_t)tri_idx(0, n) << 4, m3);
-    }
-    if ((e = cudaMemcpyToSymbol(c_one4, one4, sizeof(one4))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(c_one3, one3, sizeof(one3))) != cudaSuccess) return e;
-    k_unit_terms<<<(kCand4 + 255) / 256, 256>>>();
+    if ((e = cudaMemcpyToSymbol(g_pairs, pairs, sizeof(pairs))) != cudaSuccess) return e;
+    k_unit_terms<<<1, 256>>>();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     k_unorm_tables<<<1, 256>>>();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
