@@ -53,13 +53,13 @@ def check(oracle, tx, torch, fmt, blocks, masks, weights, aw):
 @pytest.mark.parametrize("weights", [PERCEPTUAL, (1.0, 1.0, 1.0), (0.0, 1.0, 0.0), (1e6, 1e-6, 3.0), (1e-6, 0.0, 2e-6)])
 @pytest.mark.parametrize("fmt", [1, 2])
 def test_weights(tx, cuda, oracle, fmt, weights, aw):
-    n = -(-wave(cuda) * 4 // 5) + 1
+    n = -(-wave(cuda) * 21 // 25) + 1
     check(oracle, tx, cuda, fmt, mixed_blocks(n, 40 + fmt), None, weights, aw)
 
 
-@pytest.mark.parametrize("waves,extra", [(0.8, 0), (0.8, 31), (1.0, 0), (2.0, -1), (2.6, 17)])
+@pytest.mark.parametrize("waves,extra", [(0.8, 0), (0.84, 31), (1.0, 0), (2.0, -1), (2.6, 17)])
 def test_counts_and_masks(tx, cuda, oracle, waves, extra):
-    n = -(-int(wave(cuda) * waves * 5) // 5) + extra
+    n = int(wave(cuda) * waves) + 1 + extra
     rng = np.random.default_rng(n)
     masks = rng.integers(0, 65536, n).astype(np.uint32)
     masks[rng.random(n) < 0.6] = 0xFFFF
@@ -73,7 +73,7 @@ def test_ragged_image(tx, cuda, oracle):
     t = cuda.from_numpy(img).cuda()
     f = tx.Format.Bc3
     n = f.compressed_size(1021, 1117)
-    assert n // 16 >= wave(cuda) * 4 // 5
+    assert n // 16 >= wave(cuda) * 21 // 25
     out = cuda.zeros(n, dtype=cuda.uint8, device="cuda")
     tx.compress_device(f, t.data_ptr(), 1021 * 4, 4, 1021, 1117, tx.Params(), out.data_ptr(), n,
                        cuda.cuda.current_stream().cuda_stream)

@@ -37,11 +37,11 @@ cudaError_t upload_cluster_lane_tables(const uint32_t lut[4][256][2]) { return u
 // Whether a launch of n blocks goes to this kernel.
 //   Size: its CTAs stay for the whole launch or a third of it (one wave of SMs x
 //     512 blocks takes 110 us on noisy ramps and up to 440 us on smooth fields,
-//     full or not), so a launch that leaves a fifth of its last wave's blocks
+//     full or not), so a launch that leaves more than 16 % of its waves' blocks
 //     empty goes to the team form, which scales down (BC3 of smooth fields,
-//     team / this: 1024 x 1024, 84 % of a wave, 451 / 443 us; 900 x 900, 65 %,
-//     361 / 435; 1200 x 1200, 58 % of two, 582 / 656; 2048 x 2048, 84 % of four,
-//     1337 / 1322; of noisy ramps 195 / 110, 155 / 104, 264 / 163, 735 / 362).
+//     team / this: 1024 x 1024, 84 % of a wave, 440 / 434 us; 1000 x 1000, 80 %,
+//     421 / 445; 900 x 900, 65 %, 352 / 435; 2048 x 2048, 84 % of four, 1,322 /
+//     1,323; of noisy ramps 164 / 110, 156 / 109, 128 / 104, 621 / 361).
 //   Weights: the bounds are derived for weights of ordinary size, zero or
 //     2^-20 .. 2^20 with one of them not zero (products of smaller or larger ones
 //     leave the range where f32 rounding is relative).
@@ -56,7 +56,7 @@ bool cluster_lanes_take(int fmt, const DevParams &prm, size_t n, int sm_count) {
     }
     const size_t wave = (size_t)sm_count * 512;
     if (!any || wave == 0 || n > 0x7FFFFFFFull * kLaneThreads) return false;
-    return n >= (n + wave - 1) / wave * wave / 5 * 4;
+    return n >= (n + wave - 1) / wave * wave / 25 * 21;
 }
 
 template <int FMT>

@@ -15,9 +15,9 @@
 // same code; 408 -> 366 us) and the sweeps are rolled loops (an unrolled sweep
 // stalled on fetches for 6 of 10 cycles).
 //
-// BC3 2048x2048, noisy ramps: 735 -> 362 us (alpha-weighted 941 -> 376); the
-// smooth fields of nearly flat blocks, which take the grid filter: 1,337 ->
-// 1,322 us.
+// BC3 2048x2048, noisy ramps: 735 -> 361 us (alpha-weighted 941 -> 376); the
+// smooth fields of nearly flat blocks, which take the grid filter: 1,338 ->
+// 1,323 us.
 #pragma once
 #include "tx_colour.cuh"
 
@@ -172,8 +172,11 @@ static __constant__ uint32_t c_row_from[17] = {
 //     The reference's endpoint is (ax beta - bx gamma) / det, in f32 off by at
 //     most slope (3 (S + 10 X) + 54 W e) R, slope the larger of (3 W - u) / den
 //     and u / den, and by slope (18 X + 12 S_w e) R more if the weights are not
-//     all 1; the filter's own endpoint by slope (9 X + 32 W e) R and 170 W e for
-//     such weights.  An endpoint nearer to a rounding boundary than that is in
+//     all 1.  The filter's own endpoint, centred, is off by slope (9 X + 6 W e) R
+//     through c and the last rounding, and through its slope and sums by slope 32
+//     W D R, 202 W D for weights other than 1 (u, v and the prefix weights within
+//     24 W R and 72 W R, so den within 216 W^2 R, which moves a' by its share of
+//     a').  An endpoint nearer to a rounding boundary than all this is in
 //     doubt, and its candidate is kept.
 struct LaneBound {
     float2 qx[8], qy[8], qz[8], qw[8];  // centred prefix sums and weights, prefixes 1..16 in pairs
@@ -304,7 +307,7 @@ struct ClusterLanes {
         const float T = (cw[0] * var[0] + cw[1] * var[1] + cw[2] * var[2]) * 1.01f;
         const float kappa = 9.01f * W * rcp_fast(wmin * (W - wmin));
         const float c3[3] = {B.cx, B.cy, B.cz}, X3[3] = {s.x, s.y, s.z};
-        float e1 = 0.f, d2 = 0.f, wsum = 0.f, emax = 0.f;
+        float e1 = 0.f, d2 = 0.f, wsum = 0.f, emax = 0.f, dmax = 0.f;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             float D;
@@ -315,6 +318,7 @@ struct ClusterLanes {
             d2 += cw[c] * D * D;
             wsum += cw[c];
             emax = fmaxf(emax, e);
+            dmax = fmaxf(dmax, D);
         }
         B.base = ((cw[0] * s.x) * s.x + (cw[1] * s.y) * s.y + (cw[2] * s.z) * s.z) * iw;
         B.eps = u * e1;
@@ -324,8 +328,8 @@ struct ClusterLanes {
         B.tolp = 1024.0f * u * T + 32.0f * u * W * d2;
         const float xm = fmaxf(s.x, fmaxf(s.y, s.z));
         const bool ones = wmin == 1.0f && W == (float)(int)W && rw == 0.5f * W * (W + 1.0f) + (16.0f - W) * W;
-        const float dw = ones ? 0.0f : 18.0f * xm + (12.0f * rw + 170.0f * W) * emax;
-        B.doubt = finite ? 63.0f * u * (3.0f * (r + 13.0f * xm) + 86.0f * W * emax + dw) : 1e30f;
+        const float dw = ones ? 32.0f * W * dmax : 18.0f * xm + 12.0f * rw * emax + 202.0f * W * dmax;
+        B.doubt = finite ? 63.0f * u * (3.0f * (r + 13.0f * xm) + 60.0f * W * emax + dw) : 1e30f;
     }
 
     // Take a new least error: the gain a candidate needs for it is
@@ -630,7 +634,8 @@ struct ClusterLanes {
             } while (j <= maxc && !__any_sync(0xFFFFFFFFu, pos > kRowCap - 19));
             const bool plane = j > maxc;  // the plane is complete
             if (scout && plane) push_each(record & 0xFFFFu, i, (int)(record >> 16), pos);
-            if ((plane && (scout || __reduce_add_sync(0xFFFFFFFFu, (unsigned)pos) >= 32u)) ||
+            // (the filter's own errors tighten the cut, so a queue can fill: 32 cost 1 %)
+            if ((plane && (scout || __reduce_add_sync(0xFFFFFFFFu, (unsigned)pos) >= 192u)) ||
                 __any_sync(0xFFFFFFFFu, pos > kRowCap - 19))
                 drain(pos);
             thr = fminf(thr, fminf(best_err(), least - B.base + B.eps + B.tolp));
@@ -727,7 +732,7 @@ struct ClusterLanes {
     // Deal the CTA's columns out to its threads by kind: a warp's sweep takes as
     // long as its largest set of points, and the grid filter runs for a warp if
     // some of its blocks need it, so blocks of few points, of none and of
-    // nearly one colour go together (smooth fields: 1,400 -> 1,320 us).
+    // nearly one colour go together (smooth fields: -6 %).
     __device__ __forceinline__ void deal(int count, bool finite, const LaneGuess &g, bool flat, float4 vw) {
         sm.meta[tid] = (uint32_t)count | (finite ? 32u : 0u) | (uint32_t)g.i << 6 | (uint32_t)g.j << 11 | (uint32_t)g.k << 16;
         sm.xs[tid] = vw;
