@@ -15,7 +15,7 @@
 // same code; 408 -> 366 us) and the sweeps are rolled loops (an unrolled sweep
 // stalled on fetches for 6 of 10 cycles).
 //
-// BC3 2048x2048, noisy ramps: 735 -> 361 us (alpha-weighted 941 -> 376); the
+// BC3 2048x2048, noisy ramps: 735 -> 343 us (alpha-weighted 941 -> 358); the
 // smooth fields of nearly flat blocks, which take the grid filter: 1,338 ->
 // 1,323 us.
 #pragma once
@@ -772,7 +772,7 @@ struct ClusterLanes {
         {
             uint32_t a4[4];
             colour_set_thread<BC3>(px, mask, aw, a4, cs);
-            if (cs.count == 1) best = single_thread<BC3>(px, cs, unorm);
+            if (cs.count == 1) best = single_thread<BC3>(px, cs);
             if (cs.count < 2) cs.count = 0;
             if (cs.count) {
                 colour_points_thread(px, a4, cs, aw, unorm, sqrt_count, pt);

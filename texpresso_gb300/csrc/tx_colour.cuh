@@ -24,9 +24,11 @@
 
 namespace tx {
 
-// Single-colour tables (lib/src/colourfit/single_lut.rs): [table][target][index]
-// packed start | end << 8 | error << 16.  Tables: 0 = 5_3, 1 = 6_3, 2 = 5_4, 3 = 6_4.
-static __constant__ uint32_t c_lut[4][256][2];
+// Single-colour tables (lib/src/colourfit/single_lut.rs): [table][target], x and
+// y for the two indices, packed start | end << 8 | error << 16.  Tables: 0 = 5_3,
+// 1 = 6_3, 2 = 5_4, 3 = 6_4.  (Neighbouring blocks look up different colours, which
+// constant memory would serve one after another.)
+static __device__ uint2 g_lut[4][256];
 
 // compress3's candidate list.  Entry bits: 0-3 i (offset of S(0,i)),
 // 4-11 offset of S(i,j), 20-29 rank of (i,j) in the reference's loop order at
@@ -67,70 +69,55 @@ constexpr int kTri = tri_idx(16, 16) + 1;
 // ===========================================================================
 // Shared pieces
 
-struct Single {
-    uint32_t err;
-    float s[3], e[3];
-    uint32_t index;  // 0 or 2
-};
-
-// SingleColourFit::compute_endpoints (single.rs:58-106).
-__device__ __forceinline__ Single single_endpoints(const int (&col)[3], int t0, int t1, int t2) {
-    Single r;
-    r.err = 0xFFFFFFFFu;
-    r.index = 0;
-    r.s[0] = r.s[1] = r.s[2] = 0.0f;
-    r.e[0] = r.e[1] = r.e[2] = 0.0f;
-    const int tb[3] = {t0, t1, t2};
-#pragma unroll
-    for (int index = 0; index < 2; ++index) {
-        uint32_t src[3], err = 0;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            src[c] = c_lut[tb[c]][col[c]][index];
-            const uint32_t d = (src[c] >> 16) & 0xFFu;
-            err += d * d;
-        }
-        if (err < r.err) {
-            r.s[0] = div_rn((float)(src[0] & 0xFFu), 31.0f);
-            r.s[1] = div_rn((float)(src[1] & 0xFFu), 63.0f);
-            r.s[2] = div_rn((float)(src[2] & 0xFFu), 31.0f);
-            r.e[0] = div_rn((float)((src[0] >> 8) & 0xFFu), 31.0f);
-            r.e[1] = div_rn((float)((src[1] >> 8) & 0xFFu), 63.0f);
-            r.e[2] = div_rn((float)((src[2] >> 8) & 0xFFu), 31.0f);
-            r.index = 2u * (uint32_t)index;
-            r.err = err;
-        }
-    }
-    return r;
+// Bit i of a 16-bit mask at bits 2 i and 2 i + 1.
+__device__ __forceinline__ uint32_t both_bits(uint32_t m) {
+    m = (m | m << 8) & 0x00FF00FFu;
+    m = (m | m << 4) & 0x0F0F0F0Fu;
+    m = (m | m << 2) & 0x33333333u;
+    m = (m | m << 1) & 0x55555555u;
+    return m * 3u;
 }
 
-// 2-bit index word for "every valid pixel takes `index`, excluded pixels 3".
-__device__ __forceinline__ uint32_t uniform_indices(uint32_t valid16, uint32_t index) {
-    uint32_t w = 0;
-#pragma unroll
-    for (int p = 0; p < 16; ++p) w |= (((valid16 >> p) & 1u) ? index : 3u) << (2 * p);
-    return w;
+// SingleColourFit::compute_endpoints (single.rs:58-106) for the RGB bytes of rgb.
+// Its endpoints v / 31 and v / 63 are packed again as round(31 x) and round(63 x),
+// which is v, so they stay integers: start and end as 5:6:5, error, and index (0 or
+// 2).  The first index of the smaller error is taken.
+struct Single {
+    uint32_t err, start, end, index;
+};
+__device__ __forceinline__ Single single_endpoints(uint32_t rgb, int t5, int t6) {
+    const uint2 r = __ldg(&g_lut[t5][rgb & 0xFFu]), g = __ldg(&g_lut[t6][(rgb >> 8) & 0xFFu]),
+                b = __ldg(&g_lut[t5][(rgb >> 16) & 0xFFu]);
+    auto error = [](uint32_t x, uint32_t y, uint32_t z) {
+        x = (x >> 16) & 0xFFu; y = (y >> 16) & 0xFFu; z = (z >> 16) & 0xFFu;
+        return x * x + y * y + z * z;
+    };
+    const uint32_t e0 = error(r.x, g.x, b.x), e1 = error(r.y, g.y, b.y);
+    const bool second = e1 < e0;
+    const uint32_t x = second ? r.y : r.x, y = second ? g.y : g.x, z = second ? b.y : b.x;
+    return Single{second ? e1 : e0, (x & 0xFFu) << 11 | (y & 0xFFu) << 5 | (z & 0xFFu),
+                  ((x >> 8) & 0xFFu) << 11 | ((y >> 8) & 0xFFu) << 5 | ((z >> 8) & 0xFFu), second ? 2u : 0u};
 }
 
 // SingleColourFit + ColourFit::compress (colourfit.rs:44-60) given the colour.
+// One block in ten of a textured image has a single colour, so nearly every warp
+// of the thread-per-block kernels comes here: with divisions and float packing it
+// took a third of RangeFit's time (2048x2048, noisy ramps: BC3 RangeFit 49.4 -> 40.6
+// us, BC1 62.0 -> 43.6; BC1 IterativeClusterFit 1,336 -> 1,242).
 template <int FMT>
-__device__ __forceinline__ uint2 single_fit(const int (&col)[3], uint32_t valid16, bool transparent) {
+__device__ __forceinline__ uint2 single_fit(uint32_t rgb, uint32_t valid16, bool transparent) {
+    const uint32_t out3 = both_bits(~valid16 & 0xFFFFu);  // 3 for pixels that take no part
+    auto indices = [&](uint32_t index) { return out3 | (index ? 0xAAAAAAAAu : 0u); };
     uint32_t best_err = 0xFFFFFFFFu;
     uint2 best = make_uint2(0u, 0u);
     if (FMT == BC1) {
-        const Single f = single_endpoints(col, 0, 1, 0);  // LOOKUP_5_3, 6_3, 5_3
-        if (f.err < best_err) {
-            best = write3(pack_565(f.s[0], f.s[1], f.s[2]), pack_565(f.e[0], f.e[1], f.e[2]),
-                          uniform_indices(valid16, f.index));
-            best_err = f.err;
-        }
+        const Single f = single_endpoints(rgb, 0, 1);  // LOOKUP_5_3, 6_3, 5_3
+        best = write3(f.start, f.end, indices(f.index));
+        best_err = f.err;
     }
     if (FMT != BC1 || !transparent) {
-        const Single f = single_endpoints(col, 2, 3, 2);  // LOOKUP_5_4, 6_4, 5_4
-        if (f.err < best_err) {
-            best = write4(pack_565(f.s[0], f.s[1], f.s[2]), pack_565(f.e[0], f.e[1], f.e[2]),
-                          uniform_indices(valid16, f.index));
-        }
+        const Single f = single_endpoints(rgb, 2, 3);  // LOOKUP_5_4, 6_4, 5_4
+        if (f.err < best_err) best = write4(f.start, f.end, indices(f.index));
     }
     return best;
 }
@@ -248,14 +235,11 @@ __device__ __forceinline__ void colour_set_thread(uint32_t (&px)[16], uint32_t i
 
 // The block of a one-colour set (px as colour_set_thread leaves it).
 template <int FMT>
-__device__ __forceinline__ uint2 single_thread(const uint32_t (&px)[16], const ColourSet &cs, const float *s_unorm) {
+__device__ __forceinline__ uint2 single_thread(const uint32_t (&px)[16], const ColourSet &cs) {
     uint32_t rgb = 0;
 #pragma unroll
     for (int i = 0; i < 16; ++i) rgb |= ((cs.valid >> i) & 1u) ? px[i] : 0u;
-    int col[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) col[c] = f32_to_i32_clamped(s_unorm[u8_of(rgb, c)] * 255.0f, 255);
-    return single_fit<FMT>(col, cs.valid, cs.transparent);
+    return single_fit<FMT>(rgb, cs.valid, cs.transparent);
 }
 
 // Points and weights.  Pixels that are not points get weight exactly 0,
@@ -342,7 +326,7 @@ __device__ __forceinline__ uint2 colour_range_thread(uint32_t (&px)[16], uint32_
     const uint32_t newbits = cs.newbits;
     const int count = cs.count;
     const bool transparent = cs.transparent;
-    if (count == 1) return single_thread<FMT>(px, cs, s_unorm);
+    if (count == 1) return single_thread<FMT>(px, cs);
     colour_points_thread(px, a4, cs, prm.alpha_weighted, s_unorm, s_sqrt, pt);
     float m[6];
     covariance_thread(pt, m);
@@ -1240,10 +1224,7 @@ __device__ __forceinline__ uint2 colour_cluster_team(const Team<TEAM> &tm, TeamS
 
     const uint32_t valid16 = tm.ballot(valid);
     if (count == 1) {
-        int col[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) col[c] = f32_to_i32_clamped(sm.P[c][0] * 255.0f, 255);
-        return single_fit<FMT>(col, valid16, transparent);
+        return single_fit<FMT>(tm.shfl(px & 0xFFFFFFu, __ffs(newbits) - 1), valid16, transparent);
     }
     if (count == 0) {
         // RangeFit on an empty set (range.rs:67-98): start = end = 0, error 0.
@@ -1564,7 +1545,7 @@ static inline cudaError_t upload_tables_this_tu(const uint32_t lut[4][256][2]) {
     k_unorm_tables<<<1, 256>>>();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if ((e = cudaDeviceSynchronize()) != cudaSuccess) return e;
-    return cudaMemcpyToSymbol(c_lut, lut, sizeof(uint32_t) * 4 * 256 * 2);
+    return cudaMemcpyToSymbol(g_lut, lut, sizeof(g_lut));
 }
 
 
