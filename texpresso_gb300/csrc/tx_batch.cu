@@ -47,7 +47,7 @@ cudaError_t upload_batch_tables(const uint32_t lut[4][256][2]) {
 
 __global__ void __launch_bounds__(128, 5) k_batch_lanes(BatchQueue q) {
     __shared__ float s_unorm[256];
-    __shared__ float s_sqrt[17];
+    __shared__ float s_sqrt[18];
     __shared__ float4 s_pts[16 * 128];
     init_unorm_tables(s_unorm, s_sqrt);
     const PointCol pt{s_pts + threadIdx.x, 128};

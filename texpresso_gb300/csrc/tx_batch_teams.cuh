@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_teams(BatchQueue q) {
     static_assert(STAGE >= 1 && STAGE <= 3, "staging depth");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float s_unorm[256];
-    __shared__ float s_sqrt[17];
+    __shared__ float s_sqrt[18];
     init_unorm_tables(s_unorm, s_sqrt);
     TeamSmem *teams = reinterpret_cast<TeamSmem *>(smem_raw);
     const TeamTables tt{g_cand, s_unorm, s_sqrt};

@@ -11,7 +11,7 @@ template <int FMT>
 __global__ void __launch_bounds__(128, 6) k_range(SrcDesc src, DevParams prm, uint8_t *__restrict__ out,
                                                size_t nblocks) {
     __shared__ float s_unorm[256];
-    __shared__ float s_sqrt[17];
+    __shared__ float s_sqrt[18];
     __shared__ float4 s_pts[16 * 128];
     init_unorm_tables(s_unorm, s_sqrt);
     const PointCol pt{s_pts + threadIdx.x, 128};
@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(256, 4) k_cluster(SrcDesc src, DevParams prm, 
     // 2048x2048: 742 vs 776 us); the persistent IterativeClusterFit CTAs build
     // them once and read shared memory (991 vs 999 us).
     __shared__ float s_unorm[256];
-    __shared__ float s_sqrt[17];
+    __shared__ float s_sqrt[18];
     __shared__ uint32_t s_next;
     if (NITER > 1) {
         if (threadIdx.x == 0) s_next = 0;

@@ -316,18 +316,94 @@ __device__ __forceinline__ uint32_t remap_thread(const ColourSet &cs, uint32_t c
     return out;
 }
 
+// Colour set, points and weights of RangeFit (colourset.rs:35-141).  A pixel with
+// the colour of its point gets the point's index by itself, so only the first
+// pixel of every colour (a point) and the number of its pixels are needed.
+//
+// The 120 comparisons are arithmetic: ISETP, SEL and IADD share a pipe of half the
+// rate of FADD and FFMA.  A pixel's RGB under the exponent of 2^23 or 2^24 is a
+// float of its own (pixels that take no part have others above them), so the
+// difference of two is 0, or at least 1 in size, and 1 - d^2 saturates to 1 or 0.
+// t counts the later pixels of the colour, and 32 for every earlier one.  (BC3
+// 4096x4096 128 -> 123 us, BC1 2048x2048 43.6 -> 41.6.)
+template <int FMT>
+__device__ __forceinline__ void range_points_thread(uint32_t (&px)[16], uint32_t inb, bool alpha_weighted,
+                                                    const float *s_unorm, const float *s_sqrt, const PointCol &pt,
+                                                    uint32_t &valid, uint32_t &newbits) {
+    uint32_t tbits = 0;
+    if (FMT == BC1) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) tbits |= ((px[i] >> 31) ^ 1u) << i;
+    }
+    valid = inb & ~tbits;
+    uint32_t a4[4];  // alpha of pixel 4r + c at byte c of a4[r] (alpha weighting only)
+    if (alpha_weighted) channel_words(px, 3, a4);
+    float t[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const bool in = (valid >> i) & 1u;
+        px[i] = in ? (px[i] & 0xFFFFFFu) | 0x4B000000u : 0x4C000000u | (uint32_t)i;
+        t[i] = in ? 0.0f : 32.0f;
+    }
+    auto same = [&](int i, int j) {  // 1 or 0
+        const float d = __uint_as_float(px[i]) - __uint_as_float(px[j]);
+        float e;
+        asm("fma.rn.sat.f32 %0, %1, %2, 0f3F800000;" : "=f"(e) : "f"(-d), "f"(d));
+        return e;
+    };
+    if (!alpha_weighted) {
+#pragma unroll
+        for (int i = 1; i < 16; ++i)
+#pragma unroll
+            for (int j = 0; j < i; ++j) {
+                const float e = same(i, j);
+                t[j] += e;
+                t[i] = __fmaf_rn(e, 32.0f, t[i]);
+            }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            // at most 15 later pixels; entry 17 is 0, for pixels that are no points
+            const float w = s_sqrt[1 + (int)(__float_as_uint(fminf(t[i], 16.0f) + 8388608.0f) & 31u)];
+            pt[i] = make_float4(s_unorm[u8_of(px[i], 0)], s_unorm[u8_of(px[i], 1)], s_unorm[u8_of(px[i], 2)], w);
+        }
+    } else {
+        // (a + 1) / 256 of the colour's pixels, added in pixel order, and the root
+        // (colourset.rs:69-74, :94-97); 0 of another colour's leaves the sum as it is
+        float w[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            w[i] = ((valid >> i) & 1u) ? (float)(((a4[i >> 2] >> (8 * (i & 3))) & 0xFFu) + 1u) * (1.0f / 256.0f) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < i; ++j) {
+                const float e = same(i, j);
+                w[j] = __fmaf_rn(e, w[i], w[j]);
+                t[i] = __fmaf_rn(e, 32.0f, t[i]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            pt[i] = make_float4(s_unorm[u8_of(px[i], 0)], s_unorm[u8_of(px[i], 1)], s_unorm[u8_of(px[i], 2)],
+                                t[i] < 32.0f ? sqrt_rn(w[i]) : 0.0f);
+    }
+    newbits = 0;
+#pragma unroll
+    for (int i = 15; i >= 0; --i) newbits = __funnelshift_l(__float_as_uint(t[i] - 32.0f), newbits, 1);
+}
+
 template <int FMT>
 __device__ __forceinline__ uint2 colour_range_thread(uint32_t (&px)[16], uint32_t inb,
                                                      const DevParams &prm, const float *s_unorm,
                                                      const float *s_sqrt, const PointCol &pt) {
-    uint32_t a4[4];  // alpha of pixel 4r + c at byte c of a4[r] (alpha weighting only)
-    ColourSet cs;
-    colour_set_thread<FMT>(px, inb, prm.alpha_weighted, a4, cs);
-    const uint32_t newbits = cs.newbits;
-    const int count = cs.count;
-    const bool transparent = cs.transparent;
-    if (count == 1) return single_thread<FMT>(px, cs);
-    colour_points_thread(px, a4, cs, prm.alpha_weighted, s_unorm, s_sqrt, pt);
+    uint32_t valid, newbits;
+    range_points_thread<FMT>(px, inb, prm.alpha_weighted, s_unorm, s_sqrt, pt, valid, newbits);
+    const int count = __popc(newbits);
+    const bool transparent = FMT == BC1 && valid != inb;
+    if (count == 1) {
+        uint32_t rgb = 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) rgb |= ((newbits >> i) & 1u) ? px[i] : 0u;
+        return single_fit<FMT>(rgb, valid, transparent);
+    }
     float m[6];
     covariance_thread(pt, m);
     float axis[3];
@@ -360,6 +436,85 @@ __device__ __forceinline__ uint2 colour_range_thread(uint32_t (&px)[16], uint32_
     e0 = snap(e0, 31.0f, 1.0f / 31.0f); e1 = snap(e1, 63.0f, 1.0f / 63.0f); e2 = snap(e2, 31.0f, 1.0f / 31.0f);
 
     const float w0 = prm.w[0], w1 = prm.w[1], w2 = prm.w[2];
+    const uint32_t out3 = valid == 0xFFFFu ? 0u : both_bits(~valid & 0xFFFFu);  // 3 for pixels that take no part
+    const uint32_t a565 = pack_565(s0, s1, s2), b565 = pack_565(e0, e1, e2);
+    const float c23 = 2.0f / 3.0f, c13 = 1.0f / 3.0f;
+    const float cr4[4] = {s0, e0, s0 * c23 + e0 * c13, s0 * c13 + e0 * c23};
+    const float cg4[4] = {s1, e1, s1 * c23 + e1 * c13, s1 * c13 + e1 * c23};
+    const float cb4[4] = {s2, e2, s2 * c23 + e2 * c13, s2 * c13 + e2 * c23};
+
+    // BC2 and BC3 need the nearest codes only (BC1 compares the errors of two
+    // codebooks).  The codes lie on a line, so the nearest one follows from a
+    // point's position q = g . (x - s) on it (0 at s, 1 at e): from 3 q rounded,
+    // unless that is within `near` of a rounding boundary, where the reference's own
+    // rounding decides and the point is measured.
+    //
+    // Rounding (R = 2^-24): a distance D to a code is off by 7.1 R D, and by 8 R Om
+    // sqrt(D), Om^2 = sum w^2, because codes are rounded (4 R); all D <= G^2 = sum
+    // of w_c^2 (8 var_c / wmin + 2 / 62^2) + L^2 (L the length of the line; points
+    // are within sqrt(var_c / wmin) of the mean, endpoints within half a grid step
+    // of points).  Between neighbouring codes D changes by 2 L^2 / 3 over a step, so
+    // 3 q decides but for 9 (7.1 R G^2 + 8 R Om G) / L^2, and is itself off by 3 (8
+    // R Om / L + 6 R): near = R ((64 G^2 + 100 Om G) / L^2 + 60).
+    //
+    // 9 instructions a point where measuring four codes takes 60 (BC3 2048x2048 of
+    // noisy ramps 40.6 -> 37.4 us, of smooth fields 40.6 -> 38.3).  With BC1, whose
+    // sums of distances would have to be told apart too, ramps gained as much, but
+    // smooth fields lost 20 %: there the two codebooks are often that close.
+    if (FMT != BC1) {
+        auto ordinary = [](float w) { w = fabsf(w); return w == 0.0f || (w >= 0x1p-20f && w <= 0x1p20f); };
+        const bool usual = ordinary(w0) && ordinary(w1) && ordinary(w2);
+        if (usual && a565 == b565) return write4(a565, b565, 0u);  // (which sets the indices to 0)
+        const float dr = e0 - s0, dg = e1 - s1, db = e2 - s2;
+        const float ww0 = w0 * w0, ww1 = w1 * w1, ww2 = w2 * w2;
+        const float L2 = __fmaf_rn(ww0 * dr, dr, __fmaf_rn(ww1 * dg, dg, (ww2 * db) * db));
+        const float wv = prm.alpha_weighted ? 8.1f * 16.0f : 8.1f;  // a weight is at least 1, or sqrt(1 / 256)
+        const float G2 = __fmaf_rn(ww0, __fmaf_rn(wv, m[0], 5.3e-4f), __fmaf_rn(ww1, __fmaf_rn(wv, m[3], 5.3e-4f),
+                                   __fmaf_rn(ww2, __fmaf_rn(wv, m[5], 5.3e-4f), L2)));
+        float omG, iL2;
+        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(omG) : "f"((ww0 + ww1 + ww2) * G2));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(iL2) : "f"(L2));
+        const float near = 5.9604645e-8f * __fmaf_rn(__fmaf_rn(64.0f, G2, 100.0f * omG), iL2, 60.0f);
+        if (usual && L2 > 0.0f && near < 0.25f) {
+            const float gx = ww0 * dr * iL2, gy = ww1 * dg * iL2, gz = ww2 * db * iL2;
+            const float q0 = -__fmaf_rn(gx, s0, __fmaf_rn(gy, s1, gz * s2));
+            const float M = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer
+            float pos[2] = {0.f, 0.f};    // positions in base 4
+            uint32_t todo = 0;            // bit i: point i is in doubt
+#pragma unroll
+            for (int h = 1; h >= 0; --h)
+#pragma unroll 4
+                for (int i = 8 * h + 7; i >= 8 * h; --i) {
+                    const float4 q = pt[i];
+                    const float t = __saturatef(__fmaf_rn(gx, q.x, __fmaf_rn(gy, q.y, __fmaf_rn(gz, q.z, q0))));
+                    const float k = __fmaf_rn(t, 3.0f, M) - M;
+                    pos[h] = __fmaf_rn(pos[h], 4.0f, k);
+                    todo = __funnelshift_l(__float_as_uint(0.5f - near - fabsf(__fmaf_rn(t, 3.0f, -k))), todo, 1);
+                }
+            const uint32_t p = (uint32_t)pos[0] | (uint32_t)pos[1] << 16;
+            const uint32_t hi = (p >> 1) & 0x55555555u, lo = p & 0x55555555u;
+            uint32_t closest = ((hi ^ lo) << 1) | hi;  // positions 0 .. 3 are codes 0 2 3 1
+            todo &= valid;
+#pragma unroll 1
+            while (todo) {
+                const int i = __ffs((int)todo) - 1;
+                todo &= todo - 1u;
+                const float4 q = pt[i];
+                float dist = FLT_MAX;
+                uint32_t idx = 0;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float dx = w0 * (q.x - cr4[j]), dy = w1 * (q.y - cg4[j]), dz = w2 * (q.z - cb4[j]);
+                    const float d = dx * dx + dy * dy + dz * dz;
+                    idx = d < dist ? (uint32_t)j : idx;
+                    dist = d < dist ? d : dist;
+                }
+                closest = (closest & ~(3u << (2 * i))) | idx << (2 * i);
+            }
+            return write4(a565, b565, closest | out3);
+        }
+    }
+
     float best_err = FLT_MAX;
     uint2 best = make_uint2(0u, 0u);
 
@@ -407,15 +562,13 @@ __device__ __forceinline__ uint2 colour_range_thread(uint32_t (&px)[16], uint32_
             err = err + (((newbits >> i) & 1u) ? dist : 0.0f);
         }
         if (err < best_err) {
-            const uint32_t out = remap_thread(cs, closest);
-            indices = out;
+            indices = closest | out3;
             best_err = err;
             return true;
         }
         return false;
     };
 
-    const uint32_t a565 = pack_565(s0, s1, s2), b565 = pack_565(e0, e1, e2);
     if (FMT == BC1) {
         const float cr[4] = {s0, e0, s0 * 0.5f + e0 * 0.5f, 0.0f};
         const float cg[4] = {s1, e1, s1 * 0.5f + e1 * 0.5f, 0.0f};
@@ -424,19 +577,15 @@ __device__ __forceinline__ uint2 colour_range_thread(uint32_t (&px)[16], uint32_
         if (helper(cr, cg, cb, 3, idx)) best = write3(a565, b565, idx);
     }
     if (FMT != BC1 || !transparent) {
-        const float c23 = 2.0f / 3.0f, c13 = 1.0f / 3.0f;
-        const float cr[4] = {s0, e0, s0 * c23 + e0 * c13, s0 * c13 + e0 * c23};
-        const float cg[4] = {s1, e1, s1 * c23 + e1 * c13, s1 * c13 + e1 * c23};
-        const float cb[4] = {s2, e2, s2 * c23 + e2 * c13, s2 * c13 + e2 * c23};
         uint32_t idx;
-        if (helper(cr, cg, cb, 4, idx)) best = write4(a565, b565, idx);
+        if (helper(cr4, cg4, cb4, 4, idx)) best = write4(a565, b565, idx);
     }
     return best;
 }
 
 __device__ __forceinline__ void init_unorm_tables(float *s_unorm, float *s_sqrt) {
     for (int i = threadIdx.x; i < 256; i += blockDim.x) s_unorm[i] = unorm8((uint32_t)i);
-    if (threadIdx.x < 17) s_sqrt[threadIdx.x] = sqrt_rn((float)threadIdx.x);
+    if (threadIdx.x < 18) s_sqrt[threadIdx.x] = threadIdx.x < 17 ? sqrt_rn((float)threadIdx.x) : 0.0f;
     __syncthreads();
 }
 
