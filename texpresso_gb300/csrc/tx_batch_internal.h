@@ -75,4 +75,10 @@ cudaError_t launch_batch_queues(const BatchItem *d_items, const uint2 *d_lane, u
                                 const uint32_t (&team_counts)[kTeamClasses], uint32_t team_blocks_per_unit,
                                 uint32_t *d_counters, int sm_count, const tx_batch_tuning &tuning, cudaStream_t st);
 
+// tx_batch.cu: `levels` (at most kMipChainLevels) mip levels dst of the packed RGBA8
+// image src, and a copy of it unless copy is null.
+constexpr uint32_t kMipChainLevels = 6;
+cudaError_t launch_mip_chain(const uint8_t *src, uint8_t *copy, uint32_t w, uint32_t h, uint8_t *const *dst,
+                             uint32_t levels, cudaStream_t st);
+
 }  // namespace tx

@@ -9,7 +9,7 @@
 // but no request uses) covers the request with a fixed headroom left over for
 // everything else on the device.  An admitted request gets its device memory
 // from the pool on the copy stream; its pixels are copied in and its mip chain
-// built there, overlapping the running compression steps.  Every step is one
+// built there, six levels to a launch, overlapping the running compression steps.  Every step is one
 // launch of the persistent batch kernels over a work queue assembled from all
 // ready requests: each gets a round-robin share of blocks, so requests that
 // arrive while others run join the very next step and small requests finish
@@ -98,7 +98,7 @@ struct Step {
 struct tx_server {
     tx_server_config cfg{};
     int device = 0, sm_count = 0;
-    bool host_access = false;  // kernels may write the requests' output buffers (pageable host memory)
+    bool host_access = false;  // kernels may use the requests' buffers (pageable host memory)
     cudaMemPool_t pool = nullptr;
     size_t held = 0, held_high = 0;  // bytes held by admitted requests (worker only; stats under mu)
     double busy_us = 0;              // compression-step time on the device (worker only; stats under mu)
@@ -245,14 +245,24 @@ int admit(tx_server *s) {
         q->t_admit = now_us();
         q->state = Request::LOADING;
         uint8_t *base = q->dev;
-        const Level &l0 = q->levels[0];
-        e = cudaMemcpyAsync(base + l0.src_off, q->r.rgba, (size_t)l0.w * l0.h * 4, cudaMemcpyHostToDevice, s->s_load);
-        if (e != cudaSuccess) return fail_server(e);
-        for (size_t l = 1; l < q->levels.size(); ++l) {
-            const Level &a = q->levels[l - 1], &b = q->levels[l];
-            tx_mip_job job{base + a.src_off, (size_t)a.w * 4, a.w, a.h, 4, base + b.src_off, (size_t)b.w * 4};
-            int rc = tx_mip_batch_device(&job, 1, s->s_load);
-            if (rc != TX_OK) return rc;
+        // level 0, copied or (host memory) read by the pass that makes the levels below
+        const uint8_t *src = q->r.rgba;
+        uint8_t *copy = base + q->levels[0].src_off;
+        if (!s->host_access) {
+            const Level &l0 = q->levels[0];
+            e = cudaMemcpyAsync(copy, src, (size_t)l0.w * l0.h * 4, cudaMemcpyHostToDevice, s->s_load);
+            if (e != cudaSuccess) return fail_server(e);
+            src = copy;
+            copy = nullptr;
+        }
+        for (size_t l = 0, made; copy || l + 1 < q->levels.size(); l += made) {
+            uint8_t *dst[tx::kMipChainLevels];
+            made = std::min<size_t>(q->levels.size() - 1 - l, tx::kMipChainLevels);
+            for (size_t k = 0; k < made; ++k) dst[k] = base + q->levels[l + 1 + k].src_off;
+            e = tx::launch_mip_chain(src, copy, q->levels[l].w, q->levels[l].h, dst, (uint32_t)made, s->s_load);
+            if (e != cudaSuccess) return fail_server(e);
+            src = base + q->levels[l + made].src_off;
+            copy = nullptr;
         }
         if ((e = cudaEventRecord(q->ready_ev, s->s_load)) != cudaSuccess) return fail_server(e);
         s->live.push_back(q);
@@ -464,7 +474,8 @@ void worker_main(tx_server *s) {
         if (rc == TX_OK) rc = schedule_step(s);
         if (rc == TX_OK) rc = schedule_step(s);  // keep two steps in flight
         if (rc != TX_OK) {
-            // steps and copies in flight write to the requests' outputs
+            // loads read the requests' images, steps and copies write to their outputs
+            cudaStreamSynchronize(s->s_load);
             cudaStreamSynchronize(s->s_comp);
             cudaStreamSynchronize(s->s_store);
             fail_all(s, rc);
