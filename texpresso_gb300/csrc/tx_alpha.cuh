@@ -56,11 +56,11 @@ __device__ __forceinline__ void alpha_block(const SrcDesc &src, size_t b, uint8_
     } else {
         mask = load_block_native<CH>(src, b, v0, v1);
     }
-    const uint2 r = encode_bc3_alpha(v0, mask);
+    const uint2 r = encode_bc3_alpha<true>(v0, mask);
     if (FMT == BC4) {
         __stcs(reinterpret_cast<uint2 *>(out) + b, r);
     } else {
-        const uint2 g = encode_bc3_alpha(v1, mask);
+        const uint2 g = encode_bc3_alpha<true>(v1, mask);
         __stcs(reinterpret_cast<uint4 *>(out) + b, make_uint4(r.x, r.y, g.x, g.y));
     }
 }

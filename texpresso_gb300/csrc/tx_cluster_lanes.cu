@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(kLaneThreads, 512 / kLaneThreads) k_cluster_la
     } else {
         uint32_t v[4];
         channel_words(px, 3, v);
-        al = encode_bc3_alpha(v, mask);
+        al = encode_bc3_alpha<false>(v, mask);
     }
     __syncthreads();
     const uint2 col = cl.fit(px, mask, prm.alpha_weighted, g_unorm8, g_sqrt_count);

@@ -1512,7 +1512,7 @@ __device__ __forceinline__ void range_block(const SrcDesc &src, size_t b, const 
     if (FMT == BC3) {
         uint32_t v[4];
         channel_words(px, 3, v);
-        al = encode_bc3_alpha(v, mask);
+        al = encode_bc3_alpha<false>(v, mask);
     }
     const uint2 col = colour_range_thread<FMT>(px, mask, prm, s_unorm, s_sqrt, pt);
     if (FMT == BC1) reinterpret_cast<uint2 *>(out)[b] = col;
