@@ -7,8 +7,11 @@
 
 namespace tx {
 
+// CTAs of 128 threads, ten to an SM: against 256 the last of a launch's CTAs end
+// closer together (BC4 4096x4096 24.6 -> 23.2 us, BC5 of two channels 45.7 -> 41.7;
+// of 64, a 2047x1025 BC5 took 15.1 instead of 12.5).
 template <int FMT, int CH>
-__global__ void __launch_bounds__(256) k_alpha(SrcDesc src, uint8_t *__restrict__ out, size_t nblocks) {
+__global__ void __launch_bounds__(128, 10) k_alpha(SrcDesc src, uint8_t *__restrict__ out, size_t nblocks) {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t b = (size_t)blockIdx.x * blockDim.x + threadIdx.x; b < nblocks; b += stride)
         alpha_block<FMT, CH>(src, b, out);
@@ -16,7 +19,7 @@ __global__ void __launch_bounds__(256) k_alpha(SrcDesc src, uint8_t *__restrict_
 
 template <int FMT, int CH>
 static cudaError_t launch_t(const SrcDesc &src, uint8_t *out, size_t nblocks, cudaStream_t st, const LaunchCfg &cfg) {
-    const int threads = 256;
+    const int threads = 128;
     size_t grid = (nblocks + threads - 1) / threads;
     if (grid > cfg.max_ctas) grid = cfg.max_ctas;
     if (grid == 0) grid = 1;
