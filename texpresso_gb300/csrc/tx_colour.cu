@@ -121,8 +121,18 @@ static cudaError_t launch_cluster_t(const SrcDesc &src, const DevParams &prm, ui
     // its slot without waiting for CTA partners; the slowest SM sets the
     // launch's time.  (256x256 BC1: 25.9 us in one-warp CTAs, 26.5 us in
     // 2-team and 26.9 us in 4-team CTAs.)
+    // From two waves on, BC2 and BC3 take CTAs of two teams: a CTA's slot is free
+    // when the slower of two blocks is done instead of the slowest of eight (BC3 of
+    // noisy ramps, 8 teams / 2: 400x400 33.8 / 32.9 us, 900x900 126.7 / 122.7; of
+    // smooth fields 81.5 / 78.7, 351.8 / 347.9; 280x280, one wave, 21.3 / 21.9).  BC1,
+    // whose blocks read the same code twice as long, stays with eight (1024x1024 of
+    // smooth fields 518 / 550).
     int threads = cfg.cluster_threads;
-    if (NITER == 1 && threads == 256 && nblocks < (size_t)device_sms() * 4 * (256 / TEAM)) threads = 32;
+    if (NITER == 1 && threads == 256) {
+        const size_t wave = (size_t)device_sms() * 4 * (256 / TEAM);
+        if (nblocks < wave) threads = 32;
+        else if (FMT != BC1 && nblocks >= 2 * wave) threads = 64;
+    }
     const size_t smem = cluster_smem_bytes(TEAM, threads);
     static bool attr_set[64] = {};
     int dev = 0;
