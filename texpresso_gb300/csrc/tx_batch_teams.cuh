@@ -16,11 +16,11 @@ namespace tx {
 // blocks of one level) with one atomicAdd; the blocks of the current unit and
 // then of the next units form a stream, of which the next STAGE blocks are
 // staged (pixel requested, one per lane) while the oldest one is encoded.
-// Compiled for three CTAs to an SM (80 registers) where a block's work is longest,
-// iterative BC2 and BC3, and for four elsewhere: 64 textures with all levels, half
-// of their time iterative BC3, 1,423 -> 1,348 us.
+// Compiled for three CTAs to an SM (80 registers): with the staged blocks' state,
+// 64 registers spilled and four CTAs were slower (64 textures with all levels, half
+// of their time iterative BC3, 1,420 -> 1,303 us; two CTAs 1,457 for BC2 and BC3).
 template <int TEAM, int FMT, int NITER, int STAGE>
-__global__ void __launch_bounds__(256, FMT != BC1 && NITER > 1 ? 3 : 4) k_batch_teams(BatchQueue q) {
+__global__ void __launch_bounds__(256, 3) k_batch_teams(BatchQueue q) {
     static_assert(STAGE >= 1 && STAGE <= 3, "staging depth");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float s_unorm[256];
