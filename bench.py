@@ -493,7 +493,7 @@ def run_ours(args):
     if issue is not None:
         roofline = dict(issue)
         roofline["traffic"] = int(traffic) if traffic is not None else None
-        roofline["kernel"] = "k_cluster<BC3,32,1>"
+        roofline["kernel"] = "k_cluster_lanes<BC3>"
         roofline["basis"] = ("warp instructions per launch (ncu smsp__inst_executed.sum, profiles/counters.txt, "
                              "digest %s = these sources) / this run's launch time; peak 152 SMs x 4 "
                              "sub-partitions x 1 warp instruction per clock at %.0f MHz; ncu_fma_pct = FP32 "

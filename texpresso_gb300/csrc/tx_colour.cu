@@ -119,8 +119,9 @@ static cudaError_t launch_cluster_t(const SrcDesc &src, const DevParams &prm, ui
     // in one-warp CTAs: they spread evenly over the SMs (for 4,096 blocks, 26-28
     // on an SM against 3-4 CTAs of 8 teams), and a team that finishes frees
     // its slot without waiting for CTA partners; the slowest SM sets the
-    // launch's time.  (256x256 BC1: 25.9 us in one-warp CTAs, 26.5 us in
-    // 2-team and 26.9 us in 4-team CTAs.)
+    // launch's time.  (256x256 BC1 in CTAs of 1 / 2 / 4 / 8 teams: cut-out smooth
+    // fields 25.7 / 26.3 / 27.2 / 32.2 us, noisy ramps 16.0 / 16.5 / 17.0 / 16.8,
+    // opaque ones 23.0 / 22.6 / 21.8 / 22.8.)
     // From two waves on, BC2 and BC3 take CTAs of two teams: a CTA's slot is free
     // when the slower of two blocks is done instead of the slowest of eight (BC3 of
     // noisy ramps, 8 teams / 2: 400x400 33.8 / 32.9 us, 900x900 126.7 / 122.7; of
