@@ -616,7 +616,6 @@ struct Team {
     __device__ __forceinline__ bool all(bool p) const { return __all_sync(mask, p); }
     template <class T> __device__ __forceinline__ T shfl(T v, int src) const { return __shfl_sync(mask, v, src, TEAM); }
     template <class T> __device__ __forceinline__ T shfl_up(T v, int d) const { return __shfl_up_sync(mask, v, d, TEAM); }
-    template <class T> __device__ __forceinline__ T shfl_xor(T v, int m) const { return __shfl_xor_sync(mask, v, m, TEAM); }
     __device__ __forceinline__ void sync() const { __syncwarp(mask); }
     __device__ __forceinline__ float least(float v) const {
         float r;
