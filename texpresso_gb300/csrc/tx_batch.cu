@@ -292,7 +292,7 @@ void default_tuning(tx_batch_tuning *t) {
     t->team_blocks_per_unit = 1;
     t->lane_ctas_per_sm = 3;
     t->lane_blocks_per_lane = 1;
-    t->team_blocks_in_flight = 1;
+    t->team_blocks_in_flight = tx::kDefaultStage;
 }
 
 void fill_tuning(const tx_batch_tuning *in, tx_batch_tuning *out) {
@@ -722,7 +722,7 @@ std::mutex g_noalloc_mu;
 
 // Per-device set-up, done by the first call on each device (with that device
 // current): the device address of the scratch array, the SM count and the
-// team kernel's shared-memory limit.
+// batch kernels (code, shared-memory limits).
 int noalloc_setup_device(int dev, NoallocDevice **out) {
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
     NoallocDevice &d = g_noalloc_dev[dev];
@@ -732,7 +732,7 @@ int noalloc_setup_device(int dev, NoallocDevice **out) {
         if (e != cudaSuccess) return fail_batch(e);
         if ((e = cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
             return fail_batch(e);
-        if ((e = tx::prepare_team_kernels()) != cudaSuccess) return fail_batch(e);
+        if ((e = tx::prepare_batch_kernels()) != cudaSuccess) return fail_batch(e);
         d.scratch = static_cast<unsigned char *>(ptr);
         d.ready = true;
     }
@@ -878,9 +878,10 @@ void fill_batch_item(const tx_batch_item &it, BatchItem *d) {
     else d->kind = alg == TX_ITERATIVE_CLUSTER_FIT ? KIND_CLUSTER_ITER : KIND_CLUSTER;
 }
 
-cudaError_t prepare_team_kernels() {
-    // the default staging depth, the one the allocation-free launch uses
-    return prepare_team_class_kernels<2>();
+cudaError_t prepare_batch_kernels() {
+    cudaFuncAttributes attr;
+    const cudaError_t e = cudaFuncGetAttributes(&attr, k_batch_lanes);
+    return e != cudaSuccess ? e : prepare_team_class_kernels<kDefaultStage>();
 }
 
 cudaError_t launch_team_classes(const BatchItem *d_items, const uint2 *d_team,

@@ -52,9 +52,14 @@ cudaError_t launch_team_classes(const BatchItem *d_items, const uint2 *d_team,
                                 const uint32_t (&team_counts)[kTeamClasses], uint32_t team_blocks_per_unit,
                                 uint32_t *counters, int sm_count, const tx_batch_tuning &tuning, cudaStream_t st);
 
-// Raise the shared-memory limit of every team kernel with 32-lane teams on
-// the current device (done by a plain launch on first use otherwise).
-cudaError_t prepare_team_kernels();
+// Blocks in flight per team by default: the depth that plans start with and the
+// allocation-free launch sets up and takes.
+constexpr int kDefaultStage = 1;
+
+// Load every kernel of the default tuning on the current device and raise the
+// team kernels' shared-memory limit (done by a plain launch on first use
+// otherwise).
+cudaError_t prepare_batch_kernels();
 
 // The team kernels with STAGE blocks in flight per team (1-3), one
 // translation unit each (tx_batch_stage<STAGE>.cu, tx_batch_teams.cuh):
