@@ -790,7 +790,10 @@ extern "C" int tx_batch_launch_noalloc(const tx_batch_item *items, size_t nitems
         }
     }
     setup.nitems = n;
-    // unit sizes: the defaults, doubled until both queues fit the scratch array
+    // Unit sizes, doubled until both queues fit the scratch array.  Two blocks per
+    // lane, where a plan takes one: the set-up kernel writes a level's units one
+    // after another (BC4 from RGBA8, 32 blocks to a unit / 64: 256x256 17.1 / 18.5
+    // us, 1024x1024 31.7 / 25.7, 4096x4096 257 / 153).
     uint32_t lane_span = 64, team_span = 1;
     uint32_t team_counts[tx::kTeamClasses] = {};
     auto count_units = [&](uint64_t *nl, uint64_t *nt) {

@@ -80,8 +80,9 @@ __global__ void __launch_bounds__(256, 3) k_batch_teams(BatchQueue q) {
     }
 }
 
-// The team kernels need more than 48 KB of dynamic shared memory: raise the
-// limit once per device and kernel.
+// Teams of 16 lanes need more than the 48 KB of dynamic shared memory that a
+// kernel has by default (CTAs of 256 threads): raise the limit once per device
+// and kernel.
 template <int TEAM, int FMT, int NITER, int STAGE>
 static cudaError_t class_attr() {
     static bool attr_set[64] = {};
