@@ -16,6 +16,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace fake {
@@ -32,7 +33,9 @@ struct Event {
 };
 
 inline std::recursive_mutex mu;
+inline int device = 0;                           // of 64
 inline int host_page_tables = 1;                 // cudaDevAttrPageableMemoryAccessUsesHostPageTables
+inline cudaError_t launch_error = cudaSuccess;   // cudaGetLastError after a launch
 inline std::map<std::string, int> fail_after;    // name of a call -> calls that still succeed
 inline std::map<std::string, int> calls;         // name of a call -> how often it was made
 inline std::vector<std::string> prepared;        // kernels whose attributes were set or asked for
@@ -99,18 +102,19 @@ cudaError_t __cudaPopCallConfiguration(dim3 *g, dim3 *b, size_t *smem, void *st)
     return cudaSuccess;
 }
 cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *f) { *k = (cudaKernel_t)f; return cudaSuccess; }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3, void **args, size_t, cudaStream_t st) {
-    FAKE(const std::string &name = fake::functions()[(const void *)k];
+static cudaError_t fake_launch_kernel(cudaKernel_t k, dim3 g, void **args, cudaStream_t st) {
+    return fake::call("launch", [&] { const std::string &name = fake::functions()[(const void *)k];
          fake::launched.push_back(name);
-         fake::get(st)->ops.push_back({fake::kernel_body ? fake::kernel_body(name, g, args) : nullptr, nullptr}));
+         fake::get(st)->ops.push_back({fake::kernel_body ? fake::kernel_body(name, g, args) : nullptr, nullptr}); });
+}
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3, void **args, size_t, cudaStream_t st) {
+    return fake::launch_error = fake_launch_kernel(k, g, args, st);
 }
 
-cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
-cudaError_t cudaSetDevice(int) { return cudaSuccess; }
-cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
-cudaError_t cudaGetLastError(void) {
-    return cudaSuccess;
-}
+cudaError_t cudaGetDevice(int *d) { *d = fake::device; return cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { fake::device = d; return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int *n) { *n = 64; return cudaSuccess; }
+cudaError_t cudaGetLastError(void) { return std::exchange(fake::launch_error, cudaSuccess); }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
     *v = a == cudaDevAttrMultiProcessorCount ? 152 : a == cudaDevAttrPageableMemoryAccessUsesHostPageTables ? fake::host_page_tables : 0;
     return cudaSuccess;

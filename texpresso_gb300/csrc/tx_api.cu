@@ -196,6 +196,17 @@ int finish(cudaError_t e, cudaStream_t st) {
     return e == cudaSuccess ? TX_OK : fail(e);
 }
 
+// The same for a call that used all of the device's streams: one wait, the other
+// streams joining stream 0, unless something failed.
+int finish_all(cudaError_t e, const DeviceState &d) {
+    for (int s = 1; s < kStreams && e == cudaSuccess; ++s) {
+        if ((e = cudaEventRecord(d.joined[s], d.streams[s])) == cudaSuccess)
+            e = cudaStreamWaitEvent(d.streams[0], d.joined[s], 0);
+    }
+    for (int s = 1; s < kStreams && e != cudaSuccess; ++s) cudaStreamSynchronize(d.streams[s]);
+    return finish(e, d.streams[0]);
+}
+
 // Shared validation of Format::compress arguments (lib/src/lib.rs:287-303).
 int check_compress(int format, size_t width, size_t height, size_t output_len, size_t *nblocks) {
     if (!valid_format(format)) return TX_ERR_INVALID_FORMAT;
@@ -329,7 +340,8 @@ int tx_compress(int format, const uint8_t *rgba, size_t rgba_len, size_t width, 
     if (nbands > 8 && !taper) nbands = 8;
     const size_t band_rows = (rows + nbands - 1) / nbands;
     size_t done_w = 0;
-    for (size_t r0 = 0, band = 0; r0 < rows; ++band) {
+    e = cudaSuccess;
+    for (size_t r0 = 0, band = 0; r0 < rows && e == cudaSuccess; ++band) {
         size_t r1;
         if (taper) {
             done_w += (size_t)kTaper[band];
@@ -341,9 +353,8 @@ int tx_compress(int format, const uint8_t *rgba, size_t rgba_len, size_t width, 
         // input rows of this band
         const size_t y0 = 4 * r0, y1 = (4 * r1 < height) ? 4 * r1 : height;
         if (y0 < y1) {
-            if ((e = cudaMemcpyAsync(d->d_in + y0 * pitch, rgba + y0 * pitch, (y1 - y0) * pitch,
-                                     cudaMemcpyHostToDevice, st)) != cudaSuccess)
-                return fail(e);
+            e = cudaMemcpyAsync(d->d_in + y0 * pitch, rgba + y0 * pitch, (y1 - y0) * pitch, cudaMemcpyHostToDevice, st);
+            if (e != cudaSuccess) break;
         }
         const size_t b0 = r0 * bw, b1 = (r1 * bw < nblocks) ? r1 * bw : nblocks;
         tx::SrcDesc src;
@@ -356,19 +367,12 @@ int tx_compress(int format, const uint8_t *rgba, size_t rgba_len, size_t width, 
         src.channels = 4;
         src.vec16 = (pitch % 16 == 0) ? 1 : 0;
         src.mode = 0;
-        if ((e = launch_any(format, algorithm, src, dp, d->d_out + b0 * bs, b1 - b0, st)) != cudaSuccess) return fail(e);
-        if ((e = cudaMemcpyAsync(output + b0 * bs, d->d_out + b0 * bs, (b1 - b0) * bs, cudaMemcpyDeviceToHost, st)) !=
-            cudaSuccess)
-            return fail(e);
+        e = launch_any(format, algorithm, src, dp, d->d_out + b0 * bs, b1 - b0, st);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(output + b0 * bs, d->d_out + b0 * bs, (b1 - b0) * bs, cudaMemcpyDeviceToHost, st);
         r0 = r1;
     }
-    // one wait: the other streams join stream 0
-    for (int s = 1; s < kStreams; ++s) {
-        if ((e = cudaEventRecord(d->joined[s], d->streams[s])) != cudaSuccess) return fail(e);
-        if ((e = cudaStreamWaitEvent(d->streams[0], d->joined[s], 0)) != cudaSuccess) return fail(e);
-    }
-    if ((e = cudaStreamSynchronize(d->streams[0])) != cudaSuccess) return fail(e);
-    return TX_OK;
+    return finish_all(e, *d);
 }
 
 int tx_compress_block_masked(int format, const uint8_t *rgba, uint32_t mask, const tx_params *params,
@@ -495,11 +499,10 @@ int tx_decompress(int format, const uint8_t *data, size_t data_len, size_t width
     const bool read_host = d->host_access && reinterpret_cast<uintptr_t>(data) % 8 == 0;
     const bool write_host = d->host_access && !(read_host && overlap(output, output_len, data, in_bytes));
     cudaStream_t st = d->streams[0];
-    if (!read_host) {
-        if ((e = grow(&d->d_in, &d->in_cap, in_bytes)) != cudaSuccess) return fail(e);
-        if ((e = cudaMemcpyAsync(d->d_in, data, in_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail(e);
-    }
+    if (!read_host && (e = grow(&d->d_in, &d->in_cap, in_bytes)) != cudaSuccess) return fail(e);
     if (!write_host && (e = grow(&d->d_out, &d->out_cap, output_len)) != cudaSuccess) return fail(e);
+    if (!read_host && (e = cudaMemcpyAsync(d->d_in, data, in_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess)
+        return finish(e, st);
     e = tx::launch_decode(format, read_host ? data : d->d_in, bw, rows, width, height, write_host ? output : d->d_out,
                           width * 4, output_len, st);
     // every pixel of the first img_rows rows is written; bytes past them stay untouched
