@@ -9,6 +9,12 @@
  *     never aborts the process (the reference panics where these return an
  *     error; a Rust veneer maps a negative status back to that panic);
  *   - host-buffer entry points are synchronous and thread-safe;
+ *   - host buffers are any memory of the process (pageable, page-locked, mapped
+ *     files).  Where the device uses the host's page tables, kernels work on
+ *     them in place: their pages are made present by the call, on the calling
+ *     thread (a server's jobs: on its worker), and must stay mapped until the
+ *     call returns (the job completes).  Buffers that cannot be used in place
+ *     (not aligned to a block, not ordinary memory) are copied;
  *   - *_device entry points take device pointers and a cudaStream_t (passed
  *     as void*), are stream-ordered and return after enqueueing work.
  * There is no CPU fallback: without a usable CUDA device the compute entry

@@ -135,6 +135,7 @@ cudaError_t cudaMemPoolDestroy(cudaMemPool_t) { return cudaSuccess; }
 cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *v) { *static_cast<uint64_t *>(v) = 0; return cudaSuccess; }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *) { return cudaSuccess; }
 cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) { *a = {}; return cudaSuccess; }
 cudaError_t cudaGetSymbolAddress(void **p, const void *sym) { *p = fake::variables()[sym].data(); return cudaSuccess; }
 cudaError_t cudaMemcpyToSymbol(const void *, const void *, size_t, size_t, cudaMemcpyKind) { return cudaSuccess; }
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { FAKE(memcpy(d, s, n)); }

@@ -49,4 +49,5 @@ cudaError_t launch_decode(int fmt, const uint8_t *data, size_t blocks_wide, size
 // tx_api.cu: shared device bookkeeping for every entry point
 int tx_internal_ensure_device();                // tables uploaded on the current device
 bool tx_internal_host_access();                 // kernels on the current device may use pageable host memory
+bool tx_internal_kernels_may_use(const void *p, size_t n, bool write);  // where they may: the caller's memory at p
 void tx_internal_set_last_cuda_error(int err);  // for tx_last_cuda_error()

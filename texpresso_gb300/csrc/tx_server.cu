@@ -68,6 +68,7 @@ struct Request {
     tx_server_request r{};
     std::vector<Level> levels;
     size_t footprint = 0;
+    bool read_host = false;  // the kernels read the image in host memory
     bool direct = false;     // the kernels write the output buffer themselves
     uint8_t *dev = nullptr;  // the request's device memory (from the server's pool)
     enum State { QUEUED, LOADING, ACTIVE, DRAINING, DONE } state = QUEUED;
@@ -240,17 +241,20 @@ int admit(tx_server *s) {
         nvtxRangePushA("tx_server admit");
         s->waiting.pop_front();
         q->dev = static_cast<uint8_t *>(ptr);
+        q->read_host = s->host_access && tx_internal_kernels_may_use(q->r.rgba, (size_t)q->r.width * q->r.height * 4, false);
         // Blocks are stored whole, and every level starts at a multiple of their size.
         // 24 requests with all levels: 6.59 ms with a copy per level, 4.71 without (2.59
         // with the mip chains and encoders that came later).
-        q->direct = s->host_access && reinterpret_cast<uintptr_t>(q->r.output) % tx_block_size(q->r.format) == 0;
+        const Level &last = q->levels.back();
+        q->direct = s->host_access && reinterpret_cast<uintptr_t>(q->r.output) % tx_block_size(q->r.format) == 0 &&
+                    tx_internal_kernels_may_use(q->r.output, last.out_off + last.dst_bytes, true);
         q->t_admit = now_us();
         q->state = Request::LOADING;
         uint8_t *base = q->dev;
         // level 0, copied or (host memory) read by the pass that makes the levels below
         const uint8_t *src = q->r.rgba;
         uint8_t *copy = base + q->levels[0].src_off;
-        if (!s->host_access) {
+        if (!q->read_host) {
             const Level &l0 = q->levels[0];
             e = cudaMemcpyAsync(copy, src, (size_t)l0.w * l0.h * 4, cudaMemcpyHostToDevice, s->s_load);
             if (e != cudaSuccess) return fail_server(e);
