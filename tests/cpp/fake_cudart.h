@@ -123,7 +123,7 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const
 cudaError_t cudaFuncSetAttribute(const void *f, cudaFuncAttribute, int) { FAKE(fake::prepared.push_back(fake::functions()[f])); }
 cudaError_t cudaFuncGetAttributes(cudaFuncAttributes *, const void *f) { FAKE(fake::prepared.push_back(fake::functions()[f])); }
 
-cudaError_t cudaMalloc(void **p, size_t n) { FAKE(*p = aligned_alloc(256, (n + 255) & ~(size_t)255)); }
+cudaError_t cudaMalloc(void **p, size_t n) { FAKE(*p = memset(aligned_alloc(256, (n + 255) & ~(size_t)255), 0, n)); }
 cudaError_t cudaFree(void *p) { free(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { FAKE(*p = aligned_alloc(256, (n + 255) & ~(size_t)255)); }
 cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }

@@ -11,7 +11,7 @@ import pytest
 from conftest import ROOT
 
 
-@pytest.mark.parametrize("name", ["test_noalloc_setup", "test_nothing_in_flight", "test_host_pages"])
+@pytest.mark.parametrize("name", ["test_noalloc_setup", "test_nothing_in_flight", "test_host_pages", "test_server_output"])
 def test_host_code(built, tmp_path, name):
     objects = sorted(glob.glob(os.path.join(ROOT, "texpresso_gb300", "_build", "*.o")))
     cuda = os.path.join(os.path.dirname(os.path.realpath(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc")), "..", "include")

@@ -85,5 +85,13 @@ cudaError_t launch_batch_queues(const BatchItem *d_items, const uint2 *d_lane, u
 constexpr uint32_t kMipChainLevels = 6;
 cudaError_t launch_mip_chain(const uint8_t *src, uint8_t *copy, uint32_t w, uint32_t h, uint8_t *const *dst,
                              uint32_t levels, cudaStream_t st);
+// Copy device memory to host memory that kernels may use, of any alignment.
+struct StoreJob {
+    const uint8_t *src;
+    uint8_t *dst;
+    size_t bytes;
+};
+constexpr uint32_t kStoreJobsPerLaunch = 128;  // 128 x 28 B of kernel parameters
+cudaError_t launch_store(const StoreJob *jobs, size_t njobs, cudaStream_t st);
 
 }  // namespace tx

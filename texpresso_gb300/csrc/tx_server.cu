@@ -14,12 +14,10 @@
 // queue assembled from all ready requests: each gets a round-robin share of
 // blocks, so requests that arrive while others run join the very next step and
 // small requests finish without waiting for large ones.  Two steps are kept in
-// flight; the queue of
-// step n+1 is written while step n runs.  Where the device can use pageable host
-// memory, steps write to the requests' outputs; elsewhere, and for outputs not
-// aligned to a block, a request's levels are copied back on the third stream
-// when its last blocks have been compressed.  Its memory then goes back to the
-// pool.
+// flight; the queue of step n+1 is written while step n runs.  Behind the step
+// that compresses a request's last blocks, all its levels are copied to its output
+// on the third stream, and its memory goes back to the pool.  Where the device can
+// use pageable host memory, kernels read the image and write that output.
 //
 // Each block is encoded by the same per-block code as every other entry point,
 // so a request's bytes do not depend on what else is in flight.  The loop is
@@ -60,16 +58,15 @@ constexpr size_t kHbmHeadroom = (size_t)1 << 30;
 
 struct Level {
     uint32_t w, h, nblocks;
-    size_t src_off, dst_off, dst_bytes, out_off;
+    size_t src_off, out_off;  // in the request's device memory; in its output, and from Request::out on
 };
 
 struct Request {
     uint64_t id = 0;
     tx_server_request r{};
     std::vector<Level> levels;
-    size_t footprint = 0;
-    bool read_host = false;  // the kernels read the image in host memory
-    bool direct = false;     // the kernels write the output buffer themselves
+    size_t footprint = 0, out = 0, out_bytes = 0;  // out: where its compressed levels start in dev
+    bool read_host = false, write_host = false;    // kernels use the image, the output in host memory
     uint8_t *dev = nullptr;  // the request's device memory (from the server's pool)
     enum State { QUEUED, LOADING, ACTIVE, DRAINING, DONE } state = QUEUED;
     std::vector<uint32_t> next_block;
@@ -146,18 +143,15 @@ void plan_levels(Request *q) {
         lv.nblocks = (uint32_t)(tx_num_blocks(w) * tx_num_blocks(h));
         lv.src_off = off;
         off += align_up((size_t)w * h * 4);
-        lv.dst_bytes = tx_compressed_size(r.format, w, h);
         lv.out_off = out;
-        out += lv.dst_bytes;
+        out += tx_compressed_size(r.format, w, h);
         q->levels.push_back(lv);
         w = w > 1 ? w >> 1 : 1;
         h = h > 1 ? h >> 1 : 1;
     }
-    for (Level &lv : q->levels) {
-        lv.dst_off = off;
-        off += align_up(lv.dst_bytes);
-    }
-    q->footprint = off;
+    q->out = off;
+    q->out_bytes = out;
+    q->footprint = off + align_up(out);
     q->next_block.assign(q->levels.size(), 0);
     for (const Level &lv : q->levels) q->unassigned += lv.nblocks;
 }
@@ -242,12 +236,7 @@ int admit(tx_server *s) {
         s->waiting.pop_front();
         q->dev = static_cast<uint8_t *>(ptr);
         q->read_host = s->host_access && tx_internal_kernels_may_use(q->r.rgba, (size_t)q->r.width * q->r.height * 4, false);
-        // Blocks are stored whole, and every level starts at a multiple of their size.
-        // 24 requests with all levels: 6.59 ms with a copy per level, 4.71 without (2.59
-        // with the mip chains and encoders that came later).
-        const Level &last = q->levels.back();
-        q->direct = s->host_access && reinterpret_cast<uintptr_t>(q->r.output) % tx_block_size(q->r.format) == 0 &&
-                    tx_internal_kernels_may_use(q->r.output, last.out_off + last.dst_bytes, true);
+        q->write_host = s->host_access && tx_internal_kernels_may_use(q->r.output, q->out_bytes, true);
         q->t_admit = now_us();
         q->state = Request::LOADING;
         uint8_t *base = q->dev;
@@ -310,7 +299,7 @@ int schedule_step(tx_server *s) {
             it.format = q->r.format;
             it.channels = 4;
             it.params = q->r.params;
-            it.dst = q->direct ? q->r.output + lv.out_off : q->dev + lv.dst_off;
+            it.dst = q->dev + q->out + lv.out_off;  // (every level starts at a multiple of a block)
             tx::fill_batch_item(it, &st.h_items[n_items]);
             const tx::BatchItem &d = st.h_items[n_items];
             const bool lane = d.kind == tx::KIND_ALPHA || d.kind == tx::KIND_RANGE;
@@ -356,6 +345,16 @@ int schedule_step(tx_server *s) {
                                      s->s_comp)) != cudaSuccess)
         return fail_server(e);
     if ((e = cudaEventRecord(st.done, s->s_comp)) != cudaSuccess) return fail_server(e);
+    std::vector<tx::StoreJob> stores;
+    for (Request *q : st.finishing)
+        if (q->write_host) stores.push_back(tx::StoreJob{q->dev + q->out, q->r.output, q->out_bytes});
+    if (!stores.empty()) {
+        if ((e = cudaStreamWaitEvent(s->s_store, st.done, 0)) != cudaSuccess ||
+            (e = tx::launch_store(stores.data(), stores.size(), s->s_store)) != cudaSuccess)
+            return fail_server(e);
+        for (Request *q : st.finishing)
+            if (q->write_host && (e = cudaEventRecord(q->done_ev, s->s_store)) != cudaSuccess) return fail_server(e);
+    }
     nvtxRangePop();
     st.busy = true;
     s->next_step ^= 1;
@@ -363,7 +362,7 @@ int schedule_step(tx_server *s) {
     return TX_OK;
 }
 
-// Retire finished steps: start the device->host copies of requests that are complete and need them.
+// Retire finished steps: start the device->host copies that no kernel makes.
 int retire_steps(tx_server *s) {
     for (int i = 0; i < 2; ++i) {
         Step &st = s->steps[(s->next_step + i) & 1];  // oldest first
@@ -378,15 +377,12 @@ int retire_steps(tx_server *s) {
             s->busy_us += (double)ms * 1e3;
         }
         for (Request *q : st.finishing) {
-            uint8_t *base = q->dev;
-            if ((e = cudaStreamWaitEvent(s->s_store, st.done, 0)) != cudaSuccess) return fail_server(e);
-            for (const Level &lv : q->levels) {
-                if (lv.dst_bytes == 0 || q->direct) continue;
-                if ((e = cudaMemcpyAsync(q->r.output + lv.out_off, base + lv.dst_off, lv.dst_bytes, cudaMemcpyDeviceToHost,
-                                         s->s_store)) != cudaSuccess)
+            if (!q->write_host) {  // (such a copy may hold the host up until it is done)
+                if ((e = cudaMemcpyAsync(q->r.output, q->dev + q->out, q->out_bytes, cudaMemcpyDeviceToHost, s->s_store)) !=
+                        cudaSuccess ||
+                    (e = cudaEventRecord(q->done_ev, s->s_store)) != cudaSuccess)
                     return fail_server(e);
             }
-            if ((e = cudaEventRecord(q->done_ev, s->s_store)) != cudaSuccess) return fail_server(e);
             q->state = Request::DRAINING;
         }
         st.finishing.clear();
@@ -480,7 +476,7 @@ void worker_main(tx_server *s) {
         if (rc == TX_OK) rc = schedule_step(s);
         if (rc == TX_OK) rc = schedule_step(s);  // keep two steps in flight
         if (rc != TX_OK) {
-            // loads read the requests' images, steps and copies write to their outputs
+            // loads read the requests' images, stores write to their outputs
             cudaStreamSynchronize(s->s_load);
             cudaStreamSynchronize(s->s_comp);
             cudaStreamSynchronize(s->s_store);
