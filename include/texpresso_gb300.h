@@ -14,7 +14,8 @@
  *     them in place: their pages are made present by the call, on the calling
  *     thread (a server's jobs: on its worker), and must stay mapped until the
  *     call returns (the job completes).  Buffers that cannot be used in place
- *     (not aligned to a block, not ordinary memory) are copied;
+ *     (not aligned to a block, not ordinary memory) are copied, and all are with
+ *     TX_HOST_COPIES=1 in the environment of the first call on a device;
  *   - *_device entry points take device pointers and a cudaStream_t (passed
  *     as void*), are stream-ordered and return after enqueueing work.
  * There is no CPU fallback: without a usable CUDA device the compute entry

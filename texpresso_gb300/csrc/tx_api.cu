@@ -19,6 +19,7 @@
 #include <unistd.h>
 
 #include <atomic>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 
@@ -141,7 +142,9 @@ int ensure_ready(DeviceState **out) {
     int tables = 0;
     if ((e = cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev)) != cudaSuccess)
         return fail(e);
-    d.host_access = tables != 0;
+    // (TX_HOST_COPIES=1 asks for the form with copies, which other hosts take)
+    const char *copies = getenv("TX_HOST_COPIES");
+    d.host_access = tables != 0 && !(copies && atoi(copies) == 1);
     d.ready.store(1, std::memory_order_release);
     return TX_OK;
 }
