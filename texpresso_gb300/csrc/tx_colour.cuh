@@ -791,7 +791,9 @@ __host__ __device__ __forceinline__ void decode_entry(uint32_t e, int &i, int &j
 //     minimum by at most 32 u X (|A*| + |B*|) <= 32 u f W X^2, plus rounding of
 //     the three sums, their combination and f: <= 26 u f W Z;
 // so  E_ref >= -f (sum_c w_c q_c det + Kb) - eps1  with  Kb = 2^-17 W Z and
-// eps1 = 2^-17 W sum w_c (128 u, about twice the derived terms).
+// eps1 = 2^-17 W sum w_c (128 u, about twice the derived terms) + 1e-30, for
+// weights so small that products with them leave the normal range: each is then off
+// by up to 2^-150, at most 2^30 times that in the bound.
 // A candidate whose bound exceeds an error some candidate actually reaches
 // can neither win nor tie, so the exact sweep only needs the others.  The
 // result is the reference's choice bit for bit; only the work changes.
@@ -830,7 +832,7 @@ __device__ __forceinline__ BoundBlock bound_block(const float4 xs, const float (
     z = __fmaf_rn(cw[2], xs.z * xs.z, z);
     bb.z = z;
     bb.kb = 7.62939453125e-6f * xs.w * z;                          // 2^-17 W Z
-    bb.eps1 = 7.62939453125e-6f * xs.w * (cw[0] + cw[1] + cw[2]);  // 2^-17 W sum w
+    bb.eps1 = __fmaf_rn(7.62939453125e-6f * xs.w, cw[0] + cw[1] + cw[2], 1e-30f);  // 2^-17 W sum w, + 1e-30
     return bb;
 }
 
