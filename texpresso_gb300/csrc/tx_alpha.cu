@@ -8,8 +8,9 @@
 namespace tx {
 
 // CTAs of 128 threads, ten to an SM: against 256 the last of a launch's CTAs end
-// closer together (BC4 4096x4096 24.6 -> 23.2 us, BC5 of two channels 45.7 -> 41.7;
-// of 64, a 2047x1025 BC5 took 15.1 instead of 12.5).
+// closer together (BC4 4096x4096 24.6 -> 23.2 us, BC5 of two channels 45.7 -> 41.7,
+// although its 48 registers then spill 40 bytes; of 64, a 2047x1025 BC5 took 15.1
+// instead of 12.5).
 template <int FMT, int CH>
 __global__ void __launch_bounds__(128, 10) k_alpha(SrcDesc src, uint8_t *__restrict__ out, size_t nblocks) {
     const size_t stride = (size_t)gridDim.x * blockDim.x;

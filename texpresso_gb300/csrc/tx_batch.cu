@@ -339,7 +339,9 @@ constexpr int kTeamMaxThreads = 256;  // __launch_bounds__ of the k_batch_teams 
 // One block in flight: a staged second one takes registers from the encoder and its
 // load hides behind the other teams (64 textures with all levels 1,300 / 1,277 us,
 // three smaller sets 657 / 604, 608 / 566, 512 / 472).  One block per lane: with the
-// lanes' launch the last units end closer together (1,277 / 1,255).
+// lanes' launch the last units end closer together (1,277 / 1,255).  Four CTAs per SM,
+// of which three are resident: 2 / 3 / 4 / 6 take 1,596 / 1,236 / 1,238 / 1,239 us, the
+// smaller sets 641 / 603 / 606 / 602, 609 / 568 / 562 / 564 and 504 / 476 / 471 / 470.
 void default_tuning(tx_batch_tuning *t) {
     t->team_lanes = 32;
     t->team_threads_per_cta = 256;

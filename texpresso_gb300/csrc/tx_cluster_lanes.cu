@@ -36,12 +36,13 @@ cudaError_t upload_cluster_lane_tables(const uint32_t lut[4][256][2]) { return u
 
 // Whether a launch of n blocks goes to this kernel.
 //   Size: its CTAs stay for the whole launch or a third of it (one wave of SMs x
-//     512 blocks takes 110 us on noisy ramps and up to 440 us on smooth fields,
-//     full or not), so a launch that leaves more than 16 % of its waves' blocks
-//     empty goes to the team form, which scales down (BC3 of smooth fields,
-//     team / this: 1024 x 1024, 84 % of a wave, 440 / 434 us; 1000 x 1000, 80 %,
-//     421 / 445; 900 x 900, 65 %, 352 / 435; 2048 x 2048, 84 % of four, 1,322 /
-//     1,323; of noisy ramps 164 / 110, 156 / 109, 128 / 104, 621 / 361).
+//     512 blocks takes 106 us on noisy ramps and 435 us on smooth fields, full or
+//     not), so a launch that leaves more than 16 % of its waves' blocks empty goes
+//     to the team form, which scales down.  BC3, team / this, noisy ramps: 2048 x
+//     2048 (84 % of four waves) 588 / 340 us, 1024 x 1024 (84 % of one) 155 / 106,
+//     1000 x 1000 (80 %) 147 / 106, 900 x 900 (65 %) 121 / 102; smooth fields:
+//     1,219 / 1,320, 414 / 435, 396 / 444, 332 / 430.  (The line was drawn where
+//     smooth fields broke even before the team form left out their bounds.)
 //   Weights: the bounds are derived for weights of ordinary size, zero or
 //     2^-20 .. 2^20 with one of them not zero (products of smaller or larger ones
 //     leave the range where f32 rounding is relative).

@@ -26,9 +26,10 @@ __global__ void __launch_bounds__(256, 4) k_cluster(SrcDesc src, DevParams prm, 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // The u8 -> [0,1] and sqrt(count) tables: a ClusterFit CTA (8 blocks, then
     // the next CTA) reads them from global memory through L1, because building
-    // them in shared memory cost each CTA 256 divisions and a barrier (BC3
-    // 2048x2048: 742 vs 776 us); the persistent IterativeClusterFit CTAs build
-    // them once and read shared memory (991 vs 999 us).
+    // them in shared memory costs each CTA 256 divisions and a barrier (BC1
+    // 2048x2048 785 / 824 us, BC3 900x900 121 / 138); the persistent
+    // IterativeClusterFit CTAs build them once and read shared memory (BC3
+    // 2048x2048 835 us, from global memory 838; BC1 1,249 and 1,241).
     __shared__ float s_unorm[256];
     __shared__ float s_sqrt[18];
     __shared__ uint32_t s_next;
@@ -54,9 +55,9 @@ __global__ void __launch_bounds__(256, 4) k_cluster(SrcDesc src, DevParams prm, 
     // blocks (one colour, one ordering) takes more of them instead of idling
     // until the CTA's slowest team is done, and teams working at the same time
     // still read neighbouring pixels.  For BC2/BC3 the next block's pixels are
-    // requested before the current block is encoded; BC1, whose compress3 +
-    // compress4 code already runs at the register limit, measured faster
-    // without that (163 vs 159 Mblocks/s; BC3: 254 vs 265).
+    // requested before the current block is encoded, which was faster with an
+    // earlier sweep and is slower with this one (BC3 2048x2048 835 us, 814
+    // without); BC1, at the register limit, does not (1,249 us, 1,292 with).
     auto take = [&]() {
         uint32_t k = 0;
         if (tm.lane == 0) k = atomicAdd(&s_next, 1u);
