@@ -5,9 +5,9 @@
 // through the host's own page tables at the speed of the link, so the kernels
 // work on the caller's buffers (DeviceState::host_access): one launch, no copies.
 // A pageable copy makes the host wait for everything before it, so the bands
-// below ran one after another (1024x1024 from pageable memory: BC1 RangeFit 347
-// -> 46 us, BC1 ClusterFit of a smooth field 968 -> 584; BC3 ClusterFit 2048x2048
-// 1,228 -> 396 us, from pinned memory 767 -> 392; a 64x64 BC1 RangeFit 33 -> 25).
+// below run one after another (with them / without: 1024x1024 from pageable memory:
+// BC1 RangeFit 347 / 49 us, BC1 ClusterFit of a smooth field 968 / 519; BC3 ClusterFit
+// 2048x2048 1,228 / 396 us, from pinned memory 767 / 396; a 64x64 BC1 RangeFit 33 / 23).
 // Elsewhere an image streams through the GPU in bands of block rows so that the
 // host->device copy of one band overlaps the kernel of the previous one.
 #include "texpresso_gb300.h"
@@ -201,9 +201,10 @@ cudaError_t launch_any(int format, int algorithm, const tx::SrcDesc &src, const 
 // mappings that are not memory, and every page is read once.  Where the answer is
 // no, a copy decides.  Device and managed memory has no host pages to ask for.
 // BC3 RangeFit into untouched pages, without / with this: 256x256 51 / 31 us,
-// 2048x2048 457 / 275; its decoder 61 / 35 and 1,180 / 740.  Into the same pages
-// again: 19.4 / 20.5, 108 / 114, 13.6 / 14.5 and 125 / 132.  (Small calls on copies
-// in memory of the library's own instead: 64x64 19.2 / 20.5, no better.)
+// 2048x2048 457 / 275; its decoder 61 / 35 and 1,180 / 740; from a file mapped and
+// not yet read 72 / 45 and 645 / 143.  With the same buffers again: 19.4 / 20.5, 108
+// / 114, decoder 13.6 / 14.5 and 125 / 132; one call on each of several sets, 25 / 27.
+// (Small calls on copies in memory of the library's own: 64x64 19.2 / 20.5, no better.)
 bool kernels_may_use(const void *p, size_t n, bool write) {
     if (n == 0) return true;
     static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
